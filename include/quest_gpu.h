@@ -77,7 +77,7 @@ typedef enum { QG_FRAME_ROTATING = 0, QG_FRAME_LAB = 1 } qg_frame;
 typedef enum { QG_PREC_FP64 = 0, QG_PREC_MIXED = 1 } qg_precision;
 /* QG_COEF_AUTO: the per-pair table when it takes at most half of the free
  * device memory, else on the fly.  QG_COEF_TUNED: where the table fits, the
- * first qg_run times the table kernel (its fastest variant) against the
+ * first qg_run times the table kernel against the
  * on-the-fly kernel and keeps the faster, freeing the table if it loses; the
  * two coefficient forms are algebraically equal, so results differ only in
  * the last bits (qg_get_option "coef_mode" reports the choice). */
@@ -241,11 +241,8 @@ qg_status qg_batch_run(qg_batch *b, int n_blocks);
 qg_status qg_batch_size(const qg_batch *b, int *members, int *tasks, int *blocks);
 /* Batch options: "profile" (1 = each block's kernels launched one by one
  * instead of as the graph, with CUDA events around the far-pair launch and
- * around the step launches; same results), "far_packed" (mixed-precision
- * members: 1 = the FP32 convolution with packed pairs, the default, 0 =
- * scalar; same results), "far_gmajor" (1 = each member's far tasks in
- * source-group-major order, so a thread block's warps read the same history
- * rows, the default; same results), "mid_pipe" (1 = the step launches fetch
+ * around the step launches; same results), "far_packed" and "far_gmajor" (accepted and
+ * read back; the far launch has one form), "mid_pipe" (1 = the step launches fetch
  * several mid-range pair entries per thread before summing them, which helps
  * members with long mid lists; same results), "tune_group" (1 = the next
  * run's autotuner also times source tiles per far-kernel warp, 1, 2, 4 and
@@ -260,9 +257,8 @@ qg_status qg_batch_set_option(qg_batch *b, const char *key, int value);
  * group tuned for each size class, 0 = members keep their own),
  * "tuned_far_us" (the far launch's time the batch's autotuner measured for
  * its choice, microseconds; 0 if it did not run).  The autotuner times the
- * far launch's forms that sum the same terms (far_packed for mixed members x
- * far_gmajor) at the batch's first qg_batch_run and keeps the fastest, unless
- * one was set; "autotune" (1) asks for it again at the next run. */
+ * far launch at the batch's first qg_batch_run; "autotune" (1) asks for it
+ * again at the next run. */
 qg_status qg_batch_get_option(const qg_batch *b, const char *key, int *value);
 /* Device time in milliseconds of the batch's far-pair launches and step
  * launches (each nullable), accumulated while "profile" is on. */
@@ -329,33 +325,21 @@ qg_status qg_kernel_time(qg_handle *h, int reset, double *pair_ms, int *pair_lau
  * "profile" (1 = CUDA events around the far-pair kernel and the step
  * kernels: event nodes inside the block graphs, or around each launch when
  * "graph" is 0),
- * "far_variant" (0..11: resource shape and task order of the far-pair
- *   kernel, same results; 7 and 8 are 0 and 3 with each block's warps on one
- *   source group of consecutive target tiles; the first qg_run of an FP64
- *   table handle of 512 dots or more picks the fastest of 0, 3, 5, 6, 7, 8,
- *   9, 10 and 11 (9: the table staged by bulk-copy-engine copies on an
- *   mbarrier; 10 and 11: each source's history window run staged in shared
- *   memory, in the two task orders) by timing launches of each, unless a
- *   variant was set; mixed-precision
- *   table handles choose the same way among 0, 7 (its kernel at 150
- *   registers, target-tile and source-group major) and 1, 8 (at 128);
- *   on-the-fly handles take 8 (source-group-major order, held to 3 blocks
- *   per SM; 0 and 3: target-tile major, 1: held, 7: source-group major,
- *   all with the same results); the
- *   choice is remembered for the process, and later handles of the same kind
- *   (device, size, order, frame, precision, coefficient mode) take it
- *   without timing; batch members are not timed, the batch kernel having its
- *   own),
- * "autotune" (1 = time the far-kernel variants again now; at a block
- *   boundary between runs),
- * "far_early" (1 = the default: FP64 table handles use the far kernel's
- *   first-blocks form, whatever the variant, in the blocks where some
- *   windows start before step -22: one loop for all lanes of a warp instead
- *   of two; 0 = never; same results),
- * "far_group" (source tiles each far-kernel warp sums before writing its
- *   partial, table handles; default 4, mixed precision 2 below 256 tiles;
- *   changes the summation grouping, so results change in the last bits),
- * "tune_group" (1 = the next qg_run times the far variants and then
+ * "far_variant" (0..11: accepted and read back; one far-pair kernel serves
+ *   every value.  The first qg_run of a table handle of 512 dots or more times
+ *   it unless a value was set, and "tuned_far_us" reads the time back; it is
+ *   remembered for the process, and later handles of the same kind (device,
+ *   size, order, frame, precision, coefficient mode) are not timed),
+ * "autotune" (1 = time the far kernel again now; at a block boundary between
+ *   runs),
+ * "far_early" (1 = the default: while some windows start before step -22 and
+ *   nothing but runs has written the history, those samples are read as the
+ *   zeros they are; 0 = they are skipped one by one; same results),
+ * "far_group" (source tiles per group of the far sums, table handles;
+ *   default 4, mixed precision 2 below 256 tiles; a small ensemble's groups
+ *   are cut further so that they fill the device; changes the summation
+ *   grouping, so results change in the last bits),
+ * "tune_group" (1 = the next qg_run times the far kernel with
  *   far_group 1, 2, 4 and 8 against the default and keeps the fastest;
  *   table handles; off by default because the group changes the last bits,
  *   so a tuned handle's results depend on which group won; the choice is
@@ -373,8 +357,7 @@ qg_status qg_kernel_time(qg_handle *h, int reset, double *pair_ms, int *pair_lau
  * "reset" (restart the history at step 0, main.cpp:30-36). */
 qg_status qg_set_option(qg_handle *h, const char *key, int value);
 
-/* Reads an option back: "graph", "profile", "far_variant" (the variant in
- * use, which after the first qg_run is the autotuner's choice), "block_step",
+/* Reads an option back: "graph", "profile", "far_variant", "block_step",
  * "far_group", "tune_group", "far_early", "wait_limit", "test_skip_post", "coef_mode" (QG_COEF_TABLE or
  * QG_COEF_ON_THE_FLY: the form in use), "tuned_far_us" (the far kernel's
  * launch time the autotuner measured for its choice, microseconds; 0 if it

@@ -49,10 +49,6 @@ extern "C" const char *qg_version(void) { return "quest_b200 0.1 (sm_100a)"; }
     }                                                                                        \
   } while(0)
 
-// The on-the-fly far kernel's form: source-group-major tasks, held to 3
-// blocks per SM (qg_otf.cu variant 8).
-constexpr int kOtfVariant = 8;
-
 struct qg_handle_s {
   int n = 0, n_pad = 0, nT = 0, q = 0, T = 0;
   long long nblk = 0, P = 0;
@@ -74,12 +70,10 @@ struct qg_handle_s {
   bool mixed = false;
   bool otf = false;  // coefficients computed in the far kernel (no table)
   int group = kTileGroup;  // source tiles per far-kernel warp
-  int max_groups = 0;      // source groups the partial buffer holds
+  int max_parts = 0;       // source parts the partial buffer holds
   double2 *d_ring = nullptr;
   int W = 0, stride = 0;
   double2 *d_pcr = nullptr, *d_partial = nullptr, *d_field = nullptr, *d_scratch = nullptr;
-  unsigned *d_tile_done = nullptr;
-  int nG = 0;
   int *d_fnear_ptr = nullptr, *d_fnear_idx = nullptr;  // fused: by slot, local partner
   double2 *d_fnear_coef = nullptr;
   int *d_gnear_ptr = nullptr, *d_gnear_idx = nullptr;  // general: by internal index
@@ -115,9 +109,8 @@ struct qg_handle_s {
   int next_step = 0;
   int eval_cached = -0x7fffffff;
 
-  // K-step block graphs, [traj off, traj on] + 2 for blocks whose far launch
-  // takes its first-blocks form (some windows start before step -22)
-  cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
+  // K-step block graphs by the far kernel's form, [traj off, traj on] each
+  cudaGraphExec_t graph[4] = {};
   // profiling in graph mode: kProfRing instances of the block graph, each
   // with its own events around the far kernel and around the K step kernels;
   // an instance's times are collected when it is reused, so the stream stays full
@@ -127,12 +120,15 @@ struct qg_handle_s {
   bool pev_ready = false, pending[kProfRing] = {};
   int prof_next = 0;
   bool use_graph = true;
-  int far_variant = 3;  // cp.async-staged table (see qg_far.cu); the autotuner may change it
+  int far_variant = 3;  // "far_variant": read back as set; one far kernel serves every value
   float tuned_far_ms = 0;  // far-kernel time of the autotuner's choice
   bool tune_coef = false;  // QG_COEF_TUNED: also time the on-the-fly kernel against the table
   bool tune_group = false;  // "tune_group": also time source tiles per warp 1, 2, 4, 8
-  bool far_early = true;    // "far_early": the far kernels' first-blocks form where it applies
-  bool far_nonfinite = false;  // a far pair's table coefficient is not finite (integer delay)
+  bool far_early = true;    // "far_early": the far kernel's plain form in the first blocks where it applies
+  bool far_nonfinite = false;  // a far pair's coefficient is not finite (integer delay)
+  // the ring slots of steps before -22 hold the zeros of the last reset: no
+  // caller has written history since
+  bool ring_clean = false;
   bool tune_pending = false;  // the far-kernel autotuner runs at the first qg_run
   bool profile = false;
   // first bad step as the last batch run read it (qg_bad_step answers from it
@@ -152,7 +148,9 @@ struct qg_handle_s {
   int pair_launches = 0, step_launches = 0;
   cudaEvent_t ev_chunk[2] = {nullptr, nullptr}, ev_copy[2] = {nullptr, nullptr};
 
-  FarArgs far_args(const int *d_t0, int *far_t0_out) const
+  // `groups`: source tiles per group; `parts` per group (0: far_parts' cut)
+  FarArgs far_args(const int *d_t0, int *far_t0_out) const { return far_args(d_t0, far_t0_out, group, 0); }
+  FarArgs far_args(const int *d_t0, int *far_t0_out, int groups, int parts) const
   {
     FarArgs s{};
     s.delay = d_delay;
@@ -164,31 +162,33 @@ struct qg_handle_s {
     s.ring = d_ring;
     s.partial = d_partial;
     s.field = d_field;
-    s.tile_done = d_tile_done;
     s.n_pad = n_pad;
     s.nT = nT;
-    s.nG = nG;
     s.W = W;
     s.stride = stride;
     s.q = q;
     s.frame = params.frame;
+    groups = std::min(groups, nT);  // a larger group holds the same sources
+    s.group = groups;
+    s.parts = parts > 0 ? parts : far_parts(nT, groups);
+    s.unit = (groups * kTile + s.parts - 1) / s.parts;
+    s.nP = (nT + groups - 1) / groups * s.parts;
     s.d_t0 = d_t0;
     s.far_t0_out = far_t0_out;
-    s.variant = far_variant;
-    s.gmajor = 0;
-    s.d_bad = d_ints + 2;
     s.otf = otf ? 1 : 0;
-    s.group = group;
     s.pos = d_pos;
     s.dip = d_dip;
     s.user = d_user;
-    s.cp.c0 = params.c0;
-    s.cp.dt = params.dt;
-    s.cp.mu0 = params.mu0;
-    s.cp.hbar = params.hbar;
-    s.cp.omega = params.laser_frequency;
-    s.cp.q = q;
-    s.cp.frame = params.frame;
+    s.oc.c0dt = params.c0 * params.dt;
+    s.oc.inv_c0dt = 1.0 / s.oc.c0dt;
+    s.oc.c0 = params.c0;
+    s.oc.c0_sq = params.c0 * params.c0;
+    s.oc.A = params.mu0 / (4 * M_PI * params.hbar);
+    s.oc.inv_dt = 1.0 / params.dt;
+    s.oc.inv_dt2 = s.oc.inv_dt * s.oc.inv_dt;
+    s.oc.om = params.laser_frequency;
+    s.oc.om_sq = params.laser_frequency * params.laser_frequency;
+    s.oc.half_turns = params.laser_frequency / (M_PI * params.c0);
     s.tile_lo = shard_world > 1 ? blk_lo : 0;  // 32-dot blocks are the 32-dot target tiles
     s.tile_n = shard_world > 1 ? blk_hi - blk_lo : 0;
     return s;
@@ -463,6 +463,28 @@ static size_t table_bytes(int nT, int q, bool mixed)
 // Source tiles per far-kernel warp (see create_impl).
 static int far_group(bool mixed, int nT) { return mixed && nT < 256 ? 2 : kTileGroup; }
 
+// Source tiles per group on the fly: about 16 groups.
+static int otf_group(int nT) { return (nT + 15) / 16; }
+
+static int num_parts(int nT, int group)
+{
+  group = std::min(group, nT);
+  return (nT + group - 1) / group * far_parts(nT, group);
+}
+
+// Parts the partial buffer must hold: those of the handle's group, of the
+// on-the-fly group, and for table handles of up to 512 tiles of every group
+// the "far_group" option can set (those of group g are at most (nT / g + 1)
+// x 2 g, a part being 16 sources or more, and fewer than those of group 1
+// once 600 blocks need no cut).
+static int max_parts(int nT, int group, bool otf)
+{
+  int m = std::max(num_parts(nT, group), num_parts(nT, otf_group(nT)));
+  if(!otf && nT <= 512)
+    for(int g = 1; g <= nT; ++g) m = std::max(m, num_parts(nT, g));
+  return m;
+}
+
 // Even, so every ring row starts 32-byte aligned for paired-sample loads.
 static int ring_depth(int max_delay, int q)
 {
@@ -736,10 +758,7 @@ static qg_status reset_state(qg_handle *h)
     QG_CUDA(cudaMemsetAsync(h->d_ring32w, 0, sizeof(float2) * (size_t)h->n_pad * h->stride, h->stream));
     QG_CUDA(cudaMemsetAsync(h->d_ring32d, 0, sizeof(float2) * (size_t)h->n_pad * h->stride, h->stream));
   }
-  QG_CUDA(cudaMemsetAsync(h->d_partial, 0,
-                          sizeof(double2) * (size_t)kTimeBlock * h->nG * h->n_pad, h->stream));
   QG_CUDA(cudaMemsetAsync(h->d_field, 0, sizeof(double2) * (size_t)kTimeBlock * h->n_pad, h->stream));
-  QG_CUDA(cudaMemsetAsync(h->d_tile_done, 0, sizeof(unsigned) * (size_t)h->nT, h->stream));
   launch_init_state(h->step_args(false), h->stream);
   int init[9] = {0, 0, kBadNone, 0, 0, h->max_delay, 0, 0, 0};
   QG_CUDA(cudaMemcpyAsync(h->d_ints, init, sizeof init, cudaMemcpyHostToDevice, h->stream));
@@ -747,6 +766,7 @@ static qg_status reset_state(qg_handle *h)
   h->next_step = 0;
   h->eval_cached = -0x7fffffff;
   h->far_block = -0x7fffffff;
+  h->ring_clean = true;
   return QG_OK;
 }
 
@@ -856,8 +876,6 @@ static qg_status order_for_near_groups(qg_handle *h, const qg_dot *dots, const s
   return QG_OK;
 }
 
-static qg_status autotune_far(qg_handle *h);
-
 static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, const qg_params *p,
                              const qg_weights *weights, qg_handle *h)
 {
@@ -899,7 +917,6 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
   // better), 4 from 256 tiles, where the partial sums (16 steps x groups x
   // N, FP64) would otherwise add ~13 % to the FP32 table stream
   h->group = far_group(p->precision == QG_PREC_MIXED, h->nT);
-  h->nG = (h->nT + h->group - 1) / h->group;
   h->nblk = (long long)h->nT * (h->nT + 1) / 2;
   std::vector<double> pos((size_t)h->n_pad * 3, 0.0), dip((size_t)h->n_pad * 3, 0.0);
   std::vector<double> fr(h->n_pad, 0.0), t1(h->n_pad, 1.0), t2(h->n_pad, 1.0);
@@ -941,18 +958,13 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
   QG_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const bool rule = p->coef_mode == QG_COEF_AUTO || p->coef_mode == QG_COEF_TUNED;
   h->otf = p->coef_mode == QG_COEF_ON_THE_FLY || (rule && tb > free_b / 2);
-  // on the fly: source-group-major tasks, 3 blocks per SM (measured at
-  // N = 65536: 274 against 322 ms per FP64 launch for 7, 168 against 177
-  // mixed; same sums)
-  if(h->otf) h->far_variant = kOtfVariant;
   h->tune_coef = p->coef_mode == QG_COEF_TUNED && !h->otf;
   if(!h->otf && tb > free_b * 0.9)
     return qg_fail(QG_ERR_OOM, "qg_create: coefficient table needs %zu bytes, %zu free", tb, free_b);
   if(h->otf) {
     // about 16 source groups per target tile: enough warps for the device,
     // partial sums of K x 16 x n_pad
-    h->group = (h->nT + 15) / 16;
-    h->nG = (h->nT + h->group - 1) / h->group;
+    h->group = otf_group(h->nT);
   } else {
     QG_TRY(dalloc(h, &h->d_delay, (size_t)h->nT * h->nT * kTilePairs));
     if(h->mixed)
@@ -986,7 +998,7 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
   QG_CUDA(cudaEventCreate(&e1));
   QG_CUDA(cudaEventRecord(e0, h->stream));
   if(h->otf)
-    launch_max_delay(h->d_pos, h->d_user, h->n_pad, p->c0 * p->dt, h->d_ints + 5, h->stream);
+    launch_max_delay(h->d_pos, h->d_user, h->n_pad, p->c0 * p->dt, h->d_ints + 5, h->d_u64 + 3, h->stream);
   else
     launch_table_build(ta, h->q, h->stream);
   QG_CUDA(cudaGetLastError());
@@ -1008,6 +1020,13 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
   h->near_pairs = (long long)nn[0];  // on the fly: counted from the mid list below
   h->mid_pairs = (long long)nn[1];
   h->far_nonfinite = nn[3] > 0;
+  if(h->otf) {
+    // on the fly nothing was computed yet: any non-finite input counts too
+    bool fin = std::isfinite(p->mu0 / p->hbar) && std::isfinite(p->laser_frequency);
+    for(int i = 0; i < n && fin; ++i)
+      for(int k = 0; k < 3; ++k) fin = fin && std::isfinite(dots[i].dip[k]) && std::isfinite(dots[i].pos[k]);
+    h->far_nonfinite = h->far_nonfinite || !fin;
+  }
 
   // rings and scratch.  W covers the oldest sample a far block reads
   // (t0 - max_delay - q) even when the block is recomputed up to K - 1
@@ -1020,11 +1039,9 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
     QG_TRY(dalloc(h, &h->d_ring32d, (size_t)h->n_pad * h->stride));
   }
   QG_TRY(dalloc(h, &h->d_pcr, (size_t)kPcDepth * 4 * h->n_pad));
-  // partials for the smallest group size the "far_group" option allows
-  h->max_groups = h->otf ? h->nG : (h->nT <= 512 ? h->nT : h->nG);
-  QG_TRY(dalloc(h, &h->d_partial, (size_t)kTimeBlock * h->max_groups * h->n_pad));
+  h->max_parts = max_parts(h->nT, h->group, h->otf);
+  QG_TRY(dalloc(h, &h->d_partial, (size_t)kTimeBlock * h->max_parts * h->n_pad));
   QG_TRY(dalloc(h, &h->d_field, (size_t)kTimeBlock * h->n_pad));
-  QG_TRY(dalloc(h, &h->d_tile_done, (size_t)h->nT));
   QG_TRY(dalloc(h, &h->d_scratch, (size_t)h->n_pad * 8));
   h->traj_k = traj_steps(n);
   QG_TRY(dalloc(h, &h->d_traj, (size_t)2 * h->traj_k * n * 2));
@@ -1042,17 +1059,13 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
   return QG_OK;
 }
 
-// The far-kernel autotuner.  The FP64 table path has several kernels with
-// identical arithmetic (and so identical results) but different resource
-// shapes; which one is fastest depends on N and on the device.  Each is
-// launched twice untimed (first use, clocks settling), then timed in three
-// rounds (candidates interleaved, best of the three kept), at a block start
-// past the largest delay (every tap live, as in the steady state); the
-// fastest is kept.  The history
-// is whatever the handle holds (its values do not change the work), and the
-// far field and partials are recomputed by the next run.
-static qg_status switch_to_otf(qg_handle *h);
-
+// The far-kernel autotuner: the table kernel timed once per kind of handle,
+// against the source groups ("tune_group") and the on-the-fly kernel
+// (QG_COEF_TUNED) where those are asked for.  Each candidate is launched
+// once untimed (first use, clocks settling) and then timed, at a block start
+// past the largest delay (every tap live, as in the steady state).  The
+// history is whatever the handle holds (its values do not change the work),
+// and the far field and partials are recomputed by the next run.
 static qg_status time_far(qg_handle *h, int rounds_untimed, int rounds_timed, float *best_ms)
 {
   cudaEvent_t e0, e1;
@@ -1060,7 +1073,8 @@ static qg_status time_far(qg_handle *h, int rounds_untimed, int rounds_timed, fl
   QG_CUDA(cudaEventCreate(&e1));
   float best = 1e30f;
   for(int round = 0; round < rounds_untimed + rounds_timed; ++round) {
-    const FarArgs fa = h->far_args(h->d_ints + 7, h->d_ints + 6);
+    FarArgs fa = h->far_args(h->d_ints + 7, h->d_ints + 6);
+    fa.form = kFormPlain;
     if(round < rounds_untimed) {
       launch_far(fa, h->stream);
       continue;
@@ -1075,32 +1089,8 @@ static qg_status time_far(qg_handle *h, int rounds_untimed, int rounds_timed, fl
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  QG_CUDA(cudaGetLastError());
   *best_ms = best;
-  return QG_OK;
-}
-
-// QG_COEF_TUNED: the on-the-fly kernel (its own source grouping) against the
-// table kernel's time; when it wins, the handle switches to it and frees the
-// table.
-static qg_status autotune_coef(qg_handle *h)
-{
-  const int group_t = h->group, nG_t = h->nG, variant_t = h->far_variant;
-  h->otf = true;
-  h->group = (h->nT + 15) / 16;
-  h->nG = (h->nT + h->group - 1) / h->group;
-  h->far_variant = kOtfVariant;
-  float otf_ms = 0;
-  const qg_status st = time_far(h, 2, 3, &otf_ms);
-  if(st != QG_OK || otf_ms >= h->tuned_far_ms) {
-    h->otf = false;
-    h->group = group_t;
-    h->nG = nG_t;
-    h->far_variant = variant_t;
-    return st;
-  }
-  // the on-the-fly kernel is faster: keep it, return the table's memory
-  QG_TRY(switch_to_otf(h));
-  h->tuned_far_ms = otf_ms;
   return QG_OK;
 }
 
@@ -1109,9 +1099,7 @@ static qg_status autotune_coef(qg_handle *h)
 static qg_status switch_to_otf(qg_handle *h)
 {
   h->otf = true;
-  h->far_variant = kOtfVariant;
-  h->group = (h->nT + 15) / 16;
-  h->nG = (h->nT + h->group - 1) / h->group;
+  h->group = otf_group(h->nT);
   QG_CUDA(cudaStreamSynchronize(h->stream));
   for(void *p : {(void *)h->d_delay, (void *)h->d_coef, (void *)h->d_coef32}) {
     if(!p) continue;
@@ -1126,11 +1114,30 @@ static qg_status switch_to_otf(qg_handle *h)
   return QG_OK;
 }
 
-// Source tiles per far-kernel warp (the "far_group" option): each group
-// writes one partial per target and step, and the partials are then summed
-// over groups, so the group size changes the association of the far sums
-// (results move within rounding, not bit for bit).  The search therefore
-// runs only when asked for ("tune_group"), after the variant is chosen, and
+// QG_COEF_TUNED: the on-the-fly kernel (its own source grouping) against the
+// table kernel's time; when it wins, the handle switches to it and frees the
+// table.
+static qg_status autotune_coef(qg_handle *h)
+{
+  const int group_t = h->group;
+  h->otf = true;
+  h->group = otf_group(h->nT);
+  float otf_ms = 0;
+  const qg_status st = time_far(h, 1, 3, &otf_ms);
+  if(st != QG_OK || otf_ms >= h->tuned_far_ms) {
+    h->otf = false;
+    h->group = group_t;
+    return st;
+  }
+  // the on-the-fly kernel is faster: keep it, return the table's memory
+  QG_TRY(switch_to_otf(h));
+  h->tuned_far_ms = otf_ms;
+  return QG_OK;
+}
+
+// Source tiles per group (the "far_group" option): the group changes the
+// association of the far sums (results move within rounding, not bit for
+// bit).  The search therefore runs only when asked for ("tune_group") and
 // keeps the faster of the default and each of 1, 2, 4 and 8 that the
 // handle's partial buffer holds.
 static qg_status autotune_group(qg_handle *h)
@@ -1139,85 +1146,25 @@ static qg_status autotune_group(qg_handle *h)
   int best_g = g0;
   float best = h->tuned_far_ms;
   for(int g : {1, 2, 4, 8}) {
-    if(g == g0 || (h->nT + g - 1) / g > h->max_groups) continue;
+    if(g == g0 || num_parts(h->nT, g) > h->max_parts) continue;
     h->group = g;
-    h->nG = (h->nT + g - 1) / g;
     float t = 0;
-    QG_TRY(time_far(h, 2, 3, &t));
+    QG_TRY(time_far(h, 1, 3, &t));
     if(t < best) {
       best = t;
       best_g = g;
     }
   }
   h->group = best_g;
-  h->nG = (h->nT + best_g - 1) / best_g;
   h->tuned_far_ms = best;
   return QG_OK;
 }
 
 static qg_status autotune_far(qg_handle *h)
 {
-  if(h->otf || h->nT < 16) return QG_OK;  // one kernel, or too small to matter
-  if(h->mixed) {
-    // one table kernel at two register budgets (0 and 7: 150 registers, 1
-    // and 8: 128) in two task orders (7 and 8 source-group major), the same
-    // sums; the fastest one's time is the one the coefficient choice compares
-    launch_set_int(h->d_ints + 7, h->max_delay + h->q + 2 * kTimeBlock, h->stream);
-    float best = 1e30f;
-    int best_v = 0;
-    for(int v : {0, 7, 1, 8}) {
-      h->far_variant = v;
-      float t = 0;
-      QG_TRY(time_far(h, 2, 3, &t));
-      if(t < best) {
-        best = t;
-        best_v = v;
-      }
-    }
-    h->far_variant = best_v;
-    h->tuned_far_ms = best;
-    if(h->tune_group) QG_TRY(autotune_group(h));
-    if(h->tune_coef) QG_TRY(autotune_coef(h));
-    h->far_block = -0x7fffffff;
-    h->eval_cached = -0x7fffffff;
-    return QG_OK;
-  }
-  static const int candidates[] = {0, 3, 5, 6, 7, 8, 9, 10, 11};
-  const int t_test = h->max_delay + h->q + 2 * kTimeBlock;
-  cudaEvent_t e0, e1;
-  QG_CUDA(cudaEventCreate(&e0));
-  QG_CUDA(cudaEventCreate(&e1));
-  constexpr int nc = sizeof(candidates) / sizeof(candidates[0]);
-  float t_best[nc];
-  launch_set_int(h->d_ints + 7, t_test, h->stream);
-  for(int round = 0; round < 5; ++round)
-    for(int c = 0; c < nc; ++c) {
-      h->far_variant = candidates[c];
-      const FarArgs fa = h->far_args(h->d_ints + 7, h->d_ints + 6);
-      if(round < 2) {
-        launch_far(fa, h->stream);  // untimed: first use of the kernel, clocks settling
-        continue;
-      }
-      QG_CUDA(cudaEventRecord(e0, h->stream));
-      launch_far(fa, h->stream);
-      QG_CUDA(cudaEventRecord(e1, h->stream));
-      QG_CUDA(cudaEventSynchronize(e1));
-      float ms = 0;
-      QG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-      t_best[c] = round == 2 ? ms : std::min(t_best[c], ms);
-    }
-  float best = 1e30f;
-  int best_v = candidates[0];
-  for(int c = 0; c < nc; ++c)
-    if(t_best[c] < best) {
-      best = t_best[c];
-      best_v = candidates[c];
-    }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  QG_CUDA(cudaGetLastError());
-  h->far_variant = best_v;
-  h->tuned_far_ms = best;
+  launch_set_int(h->d_ints + 7, h->max_delay + h->q + 2 * kTimeBlock, h->stream);
+  const bool search = h->tune_group || h->tune_coef;
+  QG_TRY(time_far(h, 1, search ? 3 : 1, &h->tuned_far_ms));
   if(h->tune_group) QG_TRY(autotune_group(h));
   if(h->tune_coef) QG_TRY(autotune_coef(h));
   h->far_block = -0x7fffffff;
@@ -1237,18 +1184,16 @@ struct TuneKey {
   }
 };
 struct TuneChoice {
-  int variant, group;
+  int group;
   float far_ms;
   bool otf;
 };
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneChoice> g_tune;
 
-static qg_status switch_to_otf(qg_handle *h);
-
 static qg_status autotune_cached(qg_handle *h, bool force)
 {
-  if(h->otf || h->nT < 16) return QG_OK;
+  if(h->otf || h->nT < 16) return QG_OK;  // on the fly, or too small to matter
   // the group part of the key: 0 when the group is searched, else the one set
   const TuneKey key{h->device, h->nT,  h->q, h->params.frame, h->mixed ? 1 : 0, h->tune_coef ? 1 : 0,
                     h->tune_group ? 0 : h->group};
@@ -1256,10 +1201,8 @@ static qg_status autotune_cached(qg_handle *h, bool force)
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tune.find(key);
     if(it != g_tune.end()) {
-      h->far_variant = it->second.variant;
       h->tuned_far_ms = it->second.far_ms;
       h->group = it->second.group;
-      h->nG = (h->nT + h->group - 1) / h->group;
       if(it->second.otf) QG_TRY(switch_to_otf(h));
       h->far_block = -0x7fffffff;
       h->eval_cached = -0x7fffffff;
@@ -1268,7 +1211,7 @@ static qg_status autotune_cached(qg_handle *h, bool force)
   }
   QG_TRY(autotune_far(h));
   std::lock_guard<std::mutex> lock(g_tune_mu);
-  g_tune[key] = TuneChoice{h->far_variant, h->group, h->tuned_far_ms, h->otf};
+  g_tune[key] = TuneChoice{h->group, h->tuned_far_ms, h->otf};
   return QG_OK;
 }
 
@@ -1310,14 +1253,14 @@ static void record_event(qg_handle *h, cudaEvent_t e)
     cudaEventRecord(e, h->stream);
 }
 
-// Far blocks before this step start some windows before step -22 (the far
-// kernels' first-blocks form is faster there; both forms give the same bits).
-static bool early_block(const qg_handle *h, int t0)
+// The far kernel's form for blocks from t0 on.
+static int far_form(const qg_handle *h, int t0)
 {
-  return h->far_early && !h->far_nonfinite && t0 < h->max_delay + h->q - kWindow;
+  if(t0 >= h->max_delay + h->q - kWindow) return kFormPlain;
+  return h->far_early && h->ring_clean && !h->far_nonfinite ? kFormPlain : kFormAny;
 }
 
-static void enqueue_far(qg_handle *h, int t0, bool at_boundary, cudaEvent_t ea, cudaEvent_t eb, bool early)
+static void enqueue_far(qg_handle *h, int t0, bool at_boundary, cudaEvent_t ea, cudaEvent_t eb, int form)
 {
   // at a boundary the previous block's last step kernel (or launch_steps)
   // has stored t0 in d_ints[0]; that read keeps the launch graph-capturable
@@ -1328,7 +1271,7 @@ static void enqueue_far(qg_handle *h, int t0, bool at_boundary, cudaEvent_t ea, 
   }
   if(ea) record_event(h, ea);
   FarArgs fa = h->far_args(src, h->d_ints + 6);
-  fa.early = early ? 1 : 0;
+  fa.form = form;
   launch_far(fa, h->stream);
   if(eb) record_event(h, eb);
 }
@@ -1360,7 +1303,7 @@ static qg_status capture_block(qg_handle *h, int gi, int prof, cudaGraphExec_t *
   cudaGraph_t g;
   QG_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   enqueue_far(h, 0, true, prof >= 0 ? h->pev[prof][0] : nullptr, prof >= 0 ? h->pev[prof][1] : nullptr,
-              gi >= 2);
+              gi / 2);
   if(h->block_step)
     enqueue_step_block(h, 0, kTimeBlock, traj != 0);
   else
@@ -1459,9 +1402,9 @@ static qg_status launch_steps(qg_handle *h, int t, int count, bool traj)
     const int t0 = t - t % kTimeBlock;
     if(t == t0 && count >= kTimeBlock && h->use_graph) {
       if(h->profile) {
-        QG_TRY(launch_prof_block(h, (traj ? 1 : 0) + (early_block(h, t0) ? 2 : 0)));
+        QG_TRY(launch_prof_block(h, 2 * far_form(h, t0) + (traj ? 1 : 0)));
       } else {
-        const int gi = (traj ? 1 : 0) + (early_block(h, t0) ? 2 : 0);
+        const int gi = 2 * far_form(h, t0) + (traj ? 1 : 0);
         QG_TRY(ensure_graph(h, gi));
         QG_CUDA(cudaGraphLaunch(h->graph[gi], h->stream));
       }
@@ -1472,7 +1415,7 @@ static qg_status launch_steps(qg_handle *h, int t, int count, bool traj)
     }
     if(h->far_block != t0) {
       enqueue_far(h, t0, t == t0, h->profile ? h->ev_a[nev] : nullptr,
-                  h->profile ? h->ev_b[nev] : nullptr, early_block(h, t0));
+                  h->profile ? h->ev_b[nev] : nullptr, far_form(h, t0));
       if(h->profile) ++nev;
       h->far_block = t0;
     }
@@ -1579,7 +1522,7 @@ extern "C" qg_status qg_shard_step(qg_handle *h, double *d_slice)
   h->batch_bad_valid = false;
   const int t = h->next_step, t0 = t - t % kTimeBlock;
   if(h->far_block != t0) {
-    enqueue_far(h, t0, false, nullptr, nullptr, early_block(h, t0));
+    enqueue_far(h, t0, false, nullptr, nullptr, far_form(h, t0));
     h->far_block = t0;
   }
   enqueue_dot_step(h, t - t0, false);
@@ -1673,8 +1616,6 @@ extern "C" qg_status qg_run(qg_handle *h, int n_steps, double *rho_out, int *bad
   h->next_step = t_start + n_steps;
   if(bad == -2)
     return qg_fail(QG_ERR_CUDA, "qg_run: a wait in the step-block kernel timed out");
-  if(bad == -3)
-    return qg_fail(QG_ERR_CUDA, "qg_run: a wait for the far kernel's bulk table copies timed out");
   if(bad < 0)
     return qg_fail(QG_ERR_CUDA, "qg_run: internal scheduling error (far block or trajectory row)");
   if(bad != kBadNone) {
@@ -1694,8 +1635,8 @@ struct qg_batch_s {
   StepArgs *d_step = nullptr;
   int *d_task_off = nullptr, *d_block_off = nullptr;
   int q = -1, frame = -1, n_time = -1, mixed = 0;
-  int total_tasks = 0, total_blocks = 0;
-  int far_grid = 0;
+  int total_tasks = 0, total_blocks = 0;  // far-kernel blocks; 32-dot blocks
+  int form = kFormAny;                    // the far launch's, of the block graph
   bool dirty = true;
   cudaGraphExec_t graph = nullptr;
   int *d_bad_all = nullptr;  // members' first bad steps, gathered after each run
@@ -1703,14 +1644,10 @@ struct qg_batch_s {
   // "profile": blocks launched without the graph, CUDA events around the far
   // launch and around the block's step launches
   bool profile = false;
-  // defaults measured on B200 with the 256-ensemble workload: packed FP32
-  // pairs 17.1 against 19.7 ms per far launch, and the source-group-major
-  // order 16.3 (mixed) and 22.5 against 23.9 ms (FP64)
-  bool far_packed = true;   // mixed members: the packed FP32 convolution (same bits)
-  bool far_gmajor = true;   // members' tasks in source-group-major order (same bits)
+  // read back as set; the far launch has one form
+  bool far_packed = true, far_gmajor = true;
   bool mid_pipe = false;    // step launches stage mid entries several at a time (same bits)
-  // the far launch's forms (far_packed x far_gmajor) are timed at the first
-  // run, unless set explicitly; tuned_far_us reads the winner's time back
+  // the far launch is timed at the first run (tuned_far_us reads it back)
   bool tune_pending = true;
   float tuned_far_ms = 0;
   // "tune_group": the tuner also times source tiles per warp (1, 2, 4, 8)
@@ -1752,10 +1689,6 @@ extern "C" qg_status qg_batch_create(int capacity, qg_batch **out)
      (e = cudaMallocHost(&b->h_bad_all, sizeof(int) * capacity)) != cudaSuccess)
     return fail(qg_fail(e == cudaErrorMemoryAllocation ? QG_ERR_OOM : QG_ERR_CUDA, "qg_batch_create: %s",
                         cudaGetErrorString(e)));
-  int sms = 0, per_sm = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-  per_sm = 3;  // persistent far grid: 3 blocks of 4 warps per SM (measured best)
-  b->far_grid = std::max(1, sms * per_sm);
   *out = b;
   return QG_OK;
 }
@@ -1822,6 +1755,12 @@ extern "C" qg_status qg_batch_remove(qg_batch *b, qg_handle *h)
   return QG_OK;
 }
 
+static void batch_far(qg_batch *b)
+{
+  launch_far_batch(b->d_far, b->d_task_off, b->d_block_off, (int)b->members.size(), b->total_tasks, b->total_blocks,
+                   b->q, b->frame, b->mixed, b->form, b->stream);
+}
+
 static int size_class(int nT) { return nT < 4 ? 0 : nT < 16 ? 1 : nT < 64 ? 2 : 3; }
 
 static void drop_graphs(qg_handle *h)
@@ -1839,15 +1778,23 @@ static void drop_graphs(qg_handle *h)
       }
 }
 
+// The form that serves every member's next blocks.
+static int batch_form(const qg_batch *b)
+{
+  for(const qg_handle *h : b->members)
+    if(far_form(h, h->next_step) != kFormPlain) return kFormAny;
+  return kFormPlain;
+}
+
 static qg_status batch_rebuild(qg_batch *b)
 {
   const int n = (int)b->members.size();
+  b->form = batch_form(b);
   if(b->tune_group)
     for(qg_handle *h : b->members) {
       const int g = b->class_group[size_class(h->nT)];
-      if(g > 0 && g != h->group && !h->otf && (h->nT + g - 1) / g <= h->max_groups) {
+      if(g > 0 && g != h->group && !h->otf && num_parts(h->nT, g) <= h->max_parts) {
         h->group = g;
-        h->nG = (h->nT + g - 1) / g;
         h->far_block = -0x7fffffff;
         drop_graphs(h);
       }
@@ -1865,9 +1812,8 @@ static qg_status batch_rebuild(qg_batch *b)
   for(int e = 0; e < n; ++e) {
     qg_handle *h = b->members[e];
     fa[e] = h->far_args(h->d_ints + 0, h->d_ints + 6);
-    fa[e].gmajor = b->far_gmajor ? 1 : 0;
     sa[e] = h->step_args(false);
-    toff[e + 1] = toff[e] + h->nT * h->nG;
+    toff[e + 1] = toff[e] + far_blocks(fa[e]);
     boff[e + 1] = boff[e] + h->step_blocks;
   }
   b->total_tasks = toff[n];
@@ -1886,8 +1832,7 @@ static qg_status batch_rebuild(qg_batch *b)
   if(n > 0) {
     cudaGraph_t g;
     QG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    launch_far_batch(b->d_far, b->d_task_off, n, b->q, b->frame, b->mixed ? (b->far_packed ? 2 : 1) : 0,
-                     b->far_grid, b->stream);
+    batch_far(b);
     for(int k = 0; k < kTimeBlock; ++k)
       launch_step_batch(b->d_step, b->d_block_off, n, b->total_blocks, b->n_time, k, b->mid_pipe, b->stream);
     QG_CUDA(cudaStreamEndCapture(b->stream, &g));
@@ -1898,45 +1843,37 @@ static qg_status batch_rebuild(qg_batch *b)
   return QG_OK;
 }
 
-// The batch's autotuner: its far launch in each of the forms that sum the
-// same terms (mixed: scalar or packed FP32 pairs; both: target-tile or
-// source-group-major task order), one untimed and two timed launches each,
-// the fastest kept.  The launch recomputes the far field of every member's
-// next block from history the run has not touched yet, so timing it changes
-// nothing the run then computes.
-static qg_status batch_autotune(qg_batch *b)
+// The batch's autotuner: the far launch timed (one untimed and two timed
+// launches), and with "tune_group" each size class's source group.  The
+// launch recomputes the far field of every member's next block from history
+// the run has not touched yet, so timing it changes nothing the run then
+// computes.
+static qg_status batch_time_far(qg_batch *b, int rounds, float *best_ms)
 {
-  b->tune_pending = false;
-  const int n = (int)b->members.size();
   cudaEvent_t e0, e1;
   QG_CUDA(cudaEventCreate(&e0));
   QG_CUDA(cudaEventCreate(&e1));
-  float best = 1e30f;
-  bool best_p = b->far_packed, best_g = b->far_gmajor;
-  for(int packed = 0; packed < (b->mixed ? 2 : 1); ++packed)
-    for(int gmajor = 0; gmajor < 2; ++gmajor) {
-      b->far_packed = packed != 0;
-      b->far_gmajor = gmajor != 0;
-      QG_TRY(batch_rebuild(b));  // the members' FarArgs carry the task order
-      float t = 1e30f;
-      for(int r = 0; r < 3; ++r) {
-        QG_CUDA(cudaEventRecord(e0, b->stream));
-        launch_far_batch(b->d_far, b->d_task_off, n, b->q, b->frame, b->mixed ? (b->far_packed ? 2 : 1) : 0,
-                         b->far_grid, b->stream);
-        QG_CUDA(cudaEventRecord(e1, b->stream));
-        QG_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        QG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if(r > 0) t = std::min(t, ms);
-      }
-      if(t < best) {
-        best = t;
-        best_p = b->far_packed;
-        best_g = b->far_gmajor;
-      }
-    }
-  b->far_packed = best_p;
-  b->far_gmajor = best_g;
+  float t = 1e30f;
+  for(int r = 0; r <= rounds; ++r) {
+    QG_CUDA(cudaEventRecord(e0, b->stream));
+    batch_far(b);
+    QG_CUDA(cudaEventRecord(e1, b->stream));
+    QG_CUDA(cudaEventSynchronize(e1));
+    float ms = 0;
+    QG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    if(r > 0) t = std::min(t, ms);
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  *best_ms = t;
+  return QG_OK;
+}
+
+static qg_status batch_autotune(qg_batch *b)
+{
+  b->tune_pending = false;
+  float best = 0;
+  QG_TRY(batch_time_far(b, b->tune_group ? 2 : 1, &best));
   if(b->tune_group) {
     // one pass over the size classes present, each keeping the group that
     // made the whole launch fastest with the others fixed
@@ -1948,17 +1885,8 @@ static qg_status batch_autotune(qg_batch *b)
       for(int g : {1, 2, 4, 8}) {
         b->class_group[c] = g;
         QG_TRY(batch_rebuild(b));
-        float t = 1e30f;
-        for(int r = 0; r < 3; ++r) {
-          QG_CUDA(cudaEventRecord(e0, b->stream));
-          launch_far_batch(b->d_far, b->d_task_off, n, b->q, b->frame, b->mixed ? (b->far_packed ? 2 : 1) : 0,
-                           b->far_grid, b->stream);
-          QG_CUDA(cudaEventRecord(e1, b->stream));
-          QG_CUDA(cudaEventSynchronize(e1));
-          float ms = 0;
-          QG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-          if(r > 0) t = std::min(t, ms);
-        }
+        float t = 0;
+        QG_TRY(batch_time_far(b, 2, &t));
         if(t < best) {
           best = t;
           best_c = g;
@@ -1966,18 +1894,17 @@ static qg_status batch_autotune(qg_batch *b)
       }
       b->class_group[c] = best_c;
     }
+    QG_TRY(batch_rebuild(b));
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   b->tuned_far_ms = best;
-  return batch_rebuild(b);
+  return QG_OK;
 }
 
 extern "C" qg_status qg_batch_run(qg_batch *b, int n_blocks)
 {
   if(!b || n_blocks < 0) return qg_fail(QG_ERR_INVALID_ARG, "qg_batch_run: bad argument");
   QG_CUDA(cudaSetDevice(b->device));
-  if(b->dirty) QG_TRY(batch_rebuild(b));
+  if(b->dirty || b->form != batch_form(b)) QG_TRY(batch_rebuild(b));
   if(b->members.empty()) return QG_OK;
   if(b->tune_pending && n_blocks > 0) QG_TRY(batch_autotune(b));
   const int nm0 = (int)b->members.size();
@@ -1988,8 +1915,7 @@ extern "C" qg_status qg_batch_run(qg_batch *b, int n_blocks)
     }
     // the graph's kernels one by one, timed
     QG_CUDA(cudaEventRecord(b->ev[0], b->stream));
-    launch_far_batch(b->d_far, b->d_task_off, nm0, b->q, b->frame, b->mixed ? (b->far_packed ? 2 : 1) : 0,
-                     b->far_grid, b->stream);
+    batch_far(b);
     QG_CUDA(cudaEventRecord(b->ev[1], b->stream));
     for(int k = 0; k < kTimeBlock; ++k)
       launch_step_batch(b->d_step, b->d_block_off, nm0, b->total_blocks, b->n_time, k, b->mid_pipe, b->stream);
@@ -2034,14 +1960,10 @@ extern "C" qg_status qg_batch_set_option(qg_batch *b, const char *key, int value
   }
   if(!std::strcmp(key, "far_packed")) {
     b->far_packed = value != 0;
-    b->dirty = true;  // the block graph holds the kernel
-    b->tune_pending = false;  // an explicit choice is kept
     return QG_OK;
   }
   if(!std::strcmp(key, "far_gmajor")) {
     b->far_gmajor = value != 0;
-    b->dirty = true;
-    b->tune_pending = false;
     return QG_OK;
   }
   if(!std::strcmp(key, "autotune")) {
@@ -2205,6 +2127,19 @@ extern "C" qg_status qg_checkpoint_save(qg_handle *h, void *buf, size_t bytes)
   return QG_OK;
 }
 
+// Whether a saved ring's slots of steps from `next` on (which a run of fewer
+// than W - 22 steps shares with the steps before -22) all hold zero.
+template <typename T>
+static bool zero_from(const T *ring, int width, const qg_handle *h, int next)
+{
+  for(int i = 0; i < h->n_pad; ++i) {
+    const T *row = ring + (size_t)i * h->stride * width;
+    for(int k = next * width; k < (h->W - kWindow) * width; ++k)
+      if(row[k] != T(0)) return false;
+  }
+  return true;
+}
+
 extern "C" qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t bytes)
 {
   if(!h || !buf) return qg_fail(QG_ERR_INVALID_ARG, "qg_checkpoint_load: NULL argument");
@@ -2228,6 +2163,10 @@ extern "C" qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t by
   QG_CUDA(cudaSetDevice(h->device));
   for(int i = 0; i < qg_handle_s::kProfRing; ++i) QG_TRY(collect_prof(h, i));
   const char *p = static_cast<const char *>(buf) + sizeof hd;
+  const bool clean = zero_from(reinterpret_cast<const double *>(p), 2, h, hd.next_step) &&
+                     (!h->mixed || (zero_from(reinterpret_cast<const float *>(p + hd.ring_bytes), 2, h, hd.next_step) &&
+                                    zero_from(reinterpret_cast<const float *>(p + hd.ring_bytes + hd.ring32_bytes), 2,
+                                              h, hd.next_step)));
   QG_CUDA(cudaMemcpyAsync(h->d_ring, p, hd.ring_bytes, cudaMemcpyHostToDevice, h->stream));
   p += hd.ring_bytes;
   if(h->mixed) {
@@ -2242,6 +2181,7 @@ extern "C" qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t by
   h->next_step = hd.next_step;
   h->far_block = -0x7fffffff;
   h->eval_cached = -0x7fffffff;
+  h->ring_clean = clean;
   return QG_OK;
 }
 
@@ -2287,13 +2227,14 @@ extern "C" qg_status qg_history_evaluate(qg_handle *h, int step, const double *r
   StepArgs a = h->step_args(true);
   if(rho01_step) {
     QG_TRY(upload_io(h, rho01_step));
+    h->ring_clean = false;
     launch_ring_write(a, step, h->d_io, h->stream);
     launch_ring32_rebuild(a, h->stream);
   }
   if(h->eval_cached != step) {
-    // the far partials of [step, step + K) in the run's buffer
+    // this step's far field in the run's buffer (slice 0)
     launch_set_int(h->d_ints + 4, step, h->stream);
-    launch_far(h->far_args(h->d_ints + 4, h->d_ints + 8), h->stream);
+    launch_far_step1(h->far_args(h->d_ints + 4, h->d_ints + 8), h->stream);
     h->eval_cached = step;
     h->far_block = -0x7fffffff;
   }
@@ -2325,20 +2266,17 @@ extern "C" qg_status qg_history_evaluate_noalloc(qg_handle *h, int step, const d
   cudaStream_t s = stream ? (cudaStream_t)stream : h->stream;
   StepArgs a = h->step_args(true);
   if(d_rho01_step) {
+    h->ring_clean = false;
     launch_ring_write(a, step, (const double2 *)d_rho01_step, s);
     launch_ring32_rebuild(a, s);
     h->eval_cached = -0x7fffffff;
     h->far_block = -0x7fffffff;
   }
-  // the completion counters must start at zero; the rest is overwritten
-  QG_CUDA(cudaMemsetAsync(sc.tile_done, 0, sc.tile_bytes, s));
   launch_set_int(sc.ints + 0, step, s);
-  FarArgs fa = h->far_args(sc.ints + 0, sc.ints + 1);
-  fa.group = kTileGroup;  // the fixed scratch holds the partials of this group size
-  fa.nG = (h->nT + kTileGroup - 1) / kTileGroup;
+  // the fixed scratch holds the partials of this group size, uncut
+  FarArgs fa = h->far_args(sc.ints + 0, sc.ints + 1, kTileGroup, 1);
   fa.partial = sc.partial;
   fa.field = sc.field;
-  fa.tile_done = sc.tile_done;
   launch_far_step1(fa, s);
   a.far_field = sc.field;
   a.far_t0 = sc.ints + 0;
@@ -2363,6 +2301,7 @@ extern "C" qg_status qg_set_history(qg_handle *h, int t0, int n, const double *r
     return qg_fail(QG_ERR_INVALID_ARG, "qg_set_history: t0 = %d < -%d or n < 0", t0, kWindow);
   QG_CUDA(cudaSetDevice(h->device));
   StepArgs a = h->step_args(true);
+  if(n > 0) h->ring_clean = false;
   for(int k = 0; k < n; ++k) {
     QG_TRY(upload_io(h, rho01 + (size_t)k * h->n * 2));
     launch_ring_write(a, t0 + k, h->d_io, h->stream);
@@ -2416,8 +2355,7 @@ extern "C" qg_status qg_footprint(int n, const qg_params *p, double side, size_t
   if(!p || !bytes || n < 1) return qg_fail(QG_ERR_INVALID_ARG, "qg_footprint: bad argument");
   const int nT = (n + kTile - 1) / kTile, n_pad = nT * kTile;
   const bool otf = p->coef_mode == QG_COEF_ON_THE_FLY;
-  const int group = otf ? (nT + 15) / 16 : far_group(p->precision == QG_PREC_MIXED, nT);
-  const int nG = otf ? (nT + group - 1) / group : (nT <= 512 ? nT : (nT + group - 1) / group);
+  const int group = otf ? otf_group(nT) : far_group(p->precision == QG_PREC_MIXED, nT);
   const int q = p->interpolation_order;
   const int md = (int)std::floor(side * std::sqrt(3.0) / (p->c0 * p->dt));
   const int W = ring_depth(md, q);
@@ -2425,7 +2363,7 @@ extern "C" qg_status qg_footprint(int n, const qg_params *p, double side, size_t
   size_t b = otf ? 0 : table_bytes(nT, q, mixed);
   b += sizeof(double2) * (size_t)n_pad * (W + kRingMirror) * (mixed ? 2 : 1);
   b += sizeof(double2) * (size_t)kPcDepth * 4 * n_pad;
-  b += sizeof(double2) * (size_t)kTimeBlock * (nG + 1) * n_pad + sizeof(unsigned) * nT;
+  b += sizeof(double2) * (size_t)kTimeBlock * (max_parts(nT, group, otf) + 1) * n_pad;
   b += sizeof(double2) * (size_t)n_pad * 8;
   b += sizeof(double) * (size_t)n_pad * 9 + sizeof(int) * (size_t)n_pad * 2;
   const long long K = traj_steps(n);
@@ -2477,11 +2415,10 @@ extern "C" qg_status qg_set_option(qg_handle *h, const char *key, int value)
         return qg_fail(QG_ERR_INVALID_ARG, "qg_set_option: test_skip_post in -1 .. %d", h->step_blocks - 1);
       h->skip_post = value;
     } else if(!std::strcmp(key, "far_group")) {
-      if(h->otf || value < 1 || (h->nT + value - 1) / value > h->max_groups)
+      if(h->otf || value < 1 || (h->nT > 512 && value < far_group(h->mixed, h->nT)))
         return qg_fail(QG_ERR_INVALID_ARG, "qg_set_option: far_group %d not available (table handles, "
-                       "at least %d)", value, (h->nT + h->max_groups - 1) / std::max(h->max_groups, 1));
+                       "at least %d)", value, h->nT > 512 ? far_group(h->mixed, h->nT) : 1);
       h->group = value;
-      h->nG = (h->nT + value - 1) / value;
     } else if(!std::strcmp(key, "far_variant")) {
       if(value < 0 || value > 11) return qg_fail(QG_ERR_INVALID_ARG, "qg_set_option: far_variant in 0..11");
       h->far_variant = value;

@@ -152,103 +152,202 @@ __device__ __forceinline__ int pair_coef_ref(const double (&psrc)[3], const doub
   return fd;
 }
 
-// The same pair's floor delay and coefficients for the on-the-fly path,
-// in an algebraically equal but cheaper form (about 400 instead of about
-// 5000 instructions per pair):
-//   Lagrange weights   one reciprocal r_m = 1/(x-m) per node, then for node b
-//                      w0 = prod_{m!=b} (x-m) / prod_{m!=b} (b-m),
-//                      w1 = w0 d1 / dt, w2 = w0 (d2 + d1^2) / dt^2 with
-//                      d1 = -sum_{m!=b} r_m, d2 = -sum_{m!=b} r_m^2
-//                      (the reference's w0 d2 + w1^2 / w0 with w1 = w0 d1);
-//   dyads              contracted with the dipoles first: d_obs.(I - 3 rr).d_src
-//                      = dd - 3 (d_obs.r)(d_src.r)/r^2 and d_obs.(I - rr).d_src
-//                      = dd - (d_obs.r)(d_src.r)/r^2, so each tap needs three
-//                      real scalars G0 = (dd - 3ab/r^2) c^2/r^3,
-//                      G1 = (dd - 3ab/r^2) c/r^2, G2 = (dd - ab/r^2)/r;
+// ---- coefficients computed in the far kernel -----------------------------------
+// x / t given y = 1/t correctly rounded: q0 = x*y, the remainder x - q0*t
+// exact in one fused multiply-add, then q0 + r*y rounded once.  This is
+// Markstein's correction step (P. W. Markstein, IBM J. Res. Develop. 34(1),
+// 1990): with y within half an ulp of 1/t and q0 within one ulp of x/t it
+// returns the correctly rounded quotient, i.e. exactly x / t, barring
+// underflow and overflow.  r == 0 means q0 is exact (and keeps the sign of a
+// zero quotient).  Four independent divisions per evaluation become twelve
+// independent flops instead of four serial division sequences.
+__device__ __forceinline__ double div_by(double x, double t, double y)
+{
+  const double q0 = x * y;
+  const double r = fma(-q0, t, x);
+  return r == 0.0 ? q0 : fma(r, y, q0);
+}
+
+// 1 / x to about an ulp: the hardware's approximation (20 bits or more) and
+// one third-order Newton step, y (1 + e + e^2) with e = 1 - x y.
+__device__ __forceinline__ double rcp_newton(double x)
+{
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(fma(e, e, e), y, y);
+}
+
+// Separation, floor delay and fraction of a pair, with the operations of
+// pair_coef_ref (and of the near-pair search), so the far / mid split is the
+// table's; the division by c0 dt is div_by's, the same quotient.
+struct PairGeom {
+  double dr[3], sq, nrm, x;
+  int fd;
+};
+__device__ __forceinline__ PairGeom pair_geom(const double (&pa)[3], const double (&pb)[3], const OtfConst &o)
+{
+  PairGeom g;
+#pragma unroll
+  for(int k = 0; k < 3; ++k) g.dr[k] = pa[k] - pb[k];
+  g.sq = (g.dr[0] * g.dr[0] + g.dr[1] * g.dr[1]) + g.dr[2] * g.dr[2];
+  g.nrm = sqrt(g.sq);
+  const double late = div_by(g.nrm, o.c0dt, o.inv_c0dt);
+  const double idelay = trunc(late);
+  g.x = late - idelay;
+  g.fd = (int)idelay;
+  return g;
+}
+
+// 1 / prod_{m != b} (b - m)
+template <int Q>
+__host__ __device__ constexpr double node_scale(int b)
+{
+  double den = 1.0;
+  for(int m = 0; m <= Q; ++m)
+    if(m != b) den *= (double)(b - m);
+  return 1.0 / den;
+}
+
+// FP64 Lagrange weights at fraction x as w0, d1 and s2 with w1 = w0 d1 / dt and
+// w2 = w0 s2 / dt^2: d1 = -sum 1/(x-m) and s2 = d1^2 - sum 1/(x-m)^2 over the
+// other nodes, added in the reference's order and rounded term by term as it
+// rounds them (lagrange_set.cpp:17-41).  Near x = 0 and x = 1 those sums
+// cancel and their rounding dominates a pair's error; a form without
+// reciprocals is some 500 times more accurate there (rms over random pairs),
+// but stands as far from the table's coefficients as those are from the
+// exact ones.  Calls tap(b, w0, d1, s2) for b = 0 .. Q; x = 0 gives NaN for
+// every node but the first.
+template <int Q, class F>
+__device__ __forceinline__ void lagrange_taps(double x, const F &tap)
+{
+  double f[Q + 1], r[Q + 1], sq[Q + 1], above[Q + 1];
+#pragma unroll
+  for(int m = 0; m <= Q; ++m) {
+    f[m] = x - m;
+    r[m] = rcp_newton(f[m]);
+    sq[m] = r[m] * r[m];
+  }
+  above[Q] = 1.0;  // prod_{m > b} f_m
+#pragma unroll
+  for(int b = Q; b > 0; --b) above[b - 1] = above[b] * f[b];
+  double below = 1.0, p1 = 0.0, p2 = 0.0;  // over m < b
+#pragma unroll
+  for(int b = 0; b <= Q; ++b) {
+    double d1 = p1, d2 = p2;
+#pragma unroll
+    for(int m = b + 1; m <= Q; ++m) {
+      d1 = d1 - r[m];
+      d2 = d2 - sq[m];
+    }
+    tap(b, (below * above[b]) * node_scale<Q>(b), d1, d2 + d1 * d1);
+    below = below * f[b];
+    p1 = p1 - r[b];
+    p2 = p2 - sq[b];
+  }
+}
+
+__device__ __forceinline__ void put_tap(double2 &c, double re, double im) { c = make_double2(re, im); }
+__device__ __forceinline__ void put_tap(double &c, double re, double) { c = re; }
+
+// One pair's taps (c: complex in the rotating frame, real in
+// the lab frame), in an algebraically equal but cheaper form of
+// pair_coef_ref.  The dyads are contracted with the dipoles first:
+// d_obs.(I - 3 rr).d_src = dd - 3 (d_obs.r)(d_src.r)/r^2 and d_obs.(I - rr).d_src
+// = dd - (d_obs.r)(d_src.r)/r^2, so each tap needs three real scalars
+//   G0 = (dd - 3ab/r^2) c^2/r^3, G1 = (dd - 3ab/r^2) c/r^2, G2 = (dd - ab/r^2)/r;
 //   rotating frame     coef_i = s (G0 w0 + G1 (w1 + i om w0) + G2 (w2 + 2 i om w1
 //                      - om^2 w0)), s = -mu0/(4 pi hbar) e^{-i om r/c};
 //   lab frame          coef_i = mu0/(4 pi hbar) (G0 w0 + G1 w1 + G2 w2).
-// The floor delay uses exactly the operations of pair_coef_ref (and of the
-// near-pair search), so the far / mid split is the same as the table's; the
-// coefficients agree with the reference's to rounding.
-template <int Q>
-__device__ __forceinline__ int pair_coef_otf(const double (&psrc)[3], const double (&pobs)[3],
-                                             const double (&dsrc)[3], const double (&dobs)[3],
-                                             const CoefParams &p, double2 (&coef)[Q + 1])
+// A tap is then alpha w0 + beta w1 + gamma w2 with three factors per pair.
+// Every quantity is symmetric in the two dots to the bit, so the pair's
+// orientation does not matter.  At an integer delay the reference's weights of
+// every node but the first are NaN (lagrange_set.cpp:25-33), and so are the
+// taps.
+template <int Q, bool LAB, class C>
+__device__ __forceinline__ void pair_coef_otf(const PairGeom &g, const double (&da)[3], const double (&db)[3],
+                                              const OtfConst &o, C (&c)[Q + 1])
 {
-  double dr[3];
-#pragma unroll
-  for(int k = 0; k < 3; ++k) dr[k] = pobs[k] - psrc[k];
-  const double sq = (dr[0] * dr[0] + dr[1] * dr[1]) + dr[2] * dr[2];
-  const double nrm = sqrt(sq);
-  double idelay;
-  const double x = modf(nrm / (p.c0 * p.dt), &idelay);
-  const int fd = (int)idelay;
-
-  double xm[Q + 1], rm[Q + 1];
-#pragma unroll
-  for(int m = 0; m <= Q; ++m) {
-    xm[m] = x - m;
-    rm[m] = 1.0 / xm[m];
-  }
-  const double inv_dt = 1.0 / p.dt, inv_dt2 = inv_dt * inv_dt;
-  double w0[Q + 1], w1[Q + 1], w2[Q + 1];
-#pragma unroll
-  for(int b = 0; b <= Q; ++b) {
-    double num = 1.0, den = 1.0, d1 = 0.0, d2 = 0.0;
-#pragma unroll
-    for(int m = 0; m <= Q; ++m) {
-      if(m == b) continue;
-      num *= xm[m];
-      den *= (double)(b - m);
-      d1 -= rm[m];
-      d2 -= rm[m] * rm[m];
-    }
-    w0[b] = num / den;
-    w1[b] = (w0[b] * d1) * inv_dt;
-    w2[b] = (w0[b] * (d2 + d1 * d1)) * inv_dt2;
-  }
-
-  const double dd = (dobs[0] * dsrc[0] + dobs[1] * dsrc[1]) + dobs[2] * dsrc[2];
-  const double ar = (dobs[0] * dr[0] + dobs[1] * dr[1]) + dobs[2] * dr[2];
-  const double br = (dsrc[0] * dr[0] + dsrc[1] * dr[1]) + dsrc[2] * dr[2];
-  const double inv_r = 1.0 / nrm, inv_sq = 1.0 / sq;
+  const double dd = fma(da[2], db[2], fma(da[1], db[1], da[0] * db[0]));
+  const double ar = fma(da[2], g.dr[2], fma(da[1], g.dr[1], da[0] * g.dr[0]));
+  const double br = fma(db[2], g.dr[2], fma(db[1], g.dr[1], db[0] * g.dr[0]));
+  const double inv_r = rcp_newton(g.nrm), inv_sq = inv_r * inv_r;
   const double ab = (ar * br) * inv_sq;
-  const double g3 = dd - 3.0 * ab, g1 = dd - ab;
-  const double G0 = (g3 * (p.c0 * p.c0)) * (inv_sq * inv_r);
-  const double G1 = (g3 * p.c0) * inv_sq;
-  const double G2 = g1 * inv_r;
-  const double A = p.mu0 / (4 * M_PI * p.hbar);
-  if(p.frame == 0) {
-    const double om = p.omega;
-    double sn, cs;
-    sincos((-om * nrm) / p.c0, &sn, &cs);
-    const double2 s = make_double2(-A * cs, -A * sn);
-    const double om2 = om * om;
-#pragma unroll
-    for(int i = 0; i <= Q; ++i) {
-      const double re = (G0 * w0[i] + G1 * w1[i]) + G2 * (w2[i] - om2 * w0[i]);
-      const double im = om * (G1 * w0[i] + 2.0 * (G2 * w1[i]));
-      coef[i] = cmul(s, make_double2(re, im));
-    }
+  const double g3 = fma(-3.0, ab, dd), g1 = dd - ab;
+  const double G2 = g1 * inv_r, G1 = (g3 * o.c0) * inv_sq, G0 = (g3 * o.c0_sq) * (inv_sq * inv_r);
+  if(LAB) {
+    const double al = o.A * G0, be = (o.A * G1) * o.inv_dt, ga = (o.A * G2) * o.inv_dt2;
+    lagrange_taps<Q>(g.x, [&](int b, double w0, double d1, double s2) {
+      put_tap(c[b], w0 * fma(ga, s2, fma(be, d1, al)), 0.0);
+    });
   } else {
-#pragma unroll
-    for(int i = 0; i <= Q; ++i) coef[i] = make_double2(A * ((G0 * w0[i] + G1 * w1[i]) + G2 * w2[i]), 0.0);
+    double sn, cs;
+    sincospi(g.nrm * o.half_turns, &sn, &cs);
+    const double sx = -(o.A * cs), sy = o.A * sn;  // s = -A e^{-i pi half_turns r}
+    const double ar0 = fma(-o.om_sq, G2, G0), ai0 = o.om * G1;
+    const double br0 = G1 * o.inv_dt, bi0 = 2.0 * (o.om * G2) * o.inv_dt;
+    const double gr0 = G2 * o.inv_dt2;
+    const double alx = fma(sx, ar0, -(sy * ai0)), aly = fma(sx, ai0, sy * ar0);
+    const double bex = fma(sx, br0, -(sy * bi0)), bey = fma(sx, bi0, sy * br0);
+    const double gax = sx * gr0, gay = sy * gr0;
+    lagrange_taps<Q>(g.x, [&](int b, double w0, double d1, double s2) {
+      put_tap(c[b], w0 * fma(gax, s2, fma(bex, d1, alx)), w0 * fma(gay, s2, fma(bey, d1, aly)));
+    });
   }
-  return fd;
 }
 
-// Mixed-precision coefficients of one pair for the on-the-fly kernel.  FP64
-// is kept for the distance and the split of r / (c dt) into the floor delay
-// and the fraction x (the operations of pair_coef_otf, so the far / mid split
-// is the same), and for reducing the phase argument -omega r / c to
-// [-pi, pi]; the Lagrange weights, the dyad factors and the taps are FP32.
-//
-// Weights: with f_m = x - m and e_k the elementary symmetric polynomials of
-// {f_m : m != b}, the reference's w0 = prod f_m / den, w1 = w0 sum(-1/f_m) / dt
-// and w2 = w0 (sum(-1/f_m^2) + (sum 1/f_m)^2) / dt^2 (lagrange_set.cpp:17-41)
-// are w0 = e_Q / den, w1 = -e_{Q-1} / (den dt), w2 = 2 e_{Q-2} / (den dt^2):
-// no reciprocals, so no cancellation between 1/x-sized terms as x -> 0.
+// Lagrange node products with their first two derivatives: with
+// f_m = x - m, value = prod f_m, d1 = its derivative, h2 = half its second
+// derivative.  A node's weights (lagrange_set.cpp:17-41) leave its own factor
+// out: w0 = value / den, w1 = -d1 / (den dt), w2 = 2 h2 / (den dt^2), den =
+// prod (b - m).  Taken from the products of the factors below and above the
+// node, without reciprocals (whose 1/x-sized terms cancel as x -> 0) and at
+// six operations a node.
+template <class T>
+struct Jet {
+  T v, d, h;
+  // times the factor f = x - m
+  __device__ __forceinline__ Jet times(T f) const
+  {
+    Jet r;
+    r.v = v * f;
+    r.d = fma_(d, f, v);
+    r.h = fma_(h, f, d);
+    return r;
+  }
+  __device__ __forceinline__ Jet times(const Jet &o) const
+  {
+    Jet r;
+    r.v = v * o.v;
+    r.d = fma_(d, o.v, v * o.d);
+    r.h = fma_(h, o.v, fma_(d, o.d, v * o.h));
+    return r;
+  }
+  static __device__ __forceinline__ double fma_(double a, double b, double c) { return fma(a, b, c); }
+  static __device__ __forceinline__ float fma_(float a, float b, float c) { return fmaf(a, b, c); }
+};
+
+// calls tap(b, jet) for b = Q .. 0
+template <int Q, class T, class F>
+__device__ __forceinline__ void lagrange_jets(T x, const F &tap)
+{
+  Jet<T> below[Q + 1];  // prod_{m < b}
+  below[0] = Jet<T>{T(1), T(0), T(0)};
+#pragma unroll
+  for(int b = 0; b < Q; ++b)
+    below[b + 1] = b == 0 ? Jet<T>{x, T(1), T(0)} : below[b].times(x - T(b));
+  Jet<T> above{T(1), T(0), T(0)};  // prod_{m > b}
+#pragma unroll
+  for(int b = Q; b >= 0; --b) {
+    tap(b, b == Q ? below[b] : b == 0 ? above : below[b].times(above));
+    if(b > 0) above = b == Q ? Jet<T>{x - T(b), T(1), T(0)} : above.times(x - T(b));
+  }
+}
+
+// Mixed-precision taps of one pair.  FP64 is kept for the distance and the
+// split of r / (c dt) into the floor delay and the fraction, for 1/r, and for
+// reducing the phase omega r / c to one turn; the Lagrange weights, the dyad
+// factors and the taps are FP32.
 //
 // cf[0..Q] are the taps and cf[Q+1] their sum, taken from the identities
 // sum w0 = 1, sum w1 = sum w2 = 0 as the w0-only coefficient: the
@@ -257,92 +356,52 @@ __device__ __forceinline__ int pair_coef_otf(const double (&psrc)[3], const doub
 // FP32 rounding while the taps (each ~1e-7 relative) only meet differences.
 // An integer delay (x = 0) gives NaN taps 1..Q (and sum) and a finite tap 0,
 // as the reference's weights do, so a run turns non-finite at the same step.
-template <int Q>
-__device__ __forceinline__ int pair_coef_otf_mixed(const double (&psrc)[3], const double (&pobs)[3],
-                                                   const double (&dsrc)[3], const double (&dobs)[3],
-                                                   const CoefParams &p, float2 (&cf)[Q + 2])
+template <int Q, bool LAB>
+__device__ __forceinline__ void pair_coef_otf_mixed(const PairGeom &g, const double (&da)[3], const double (&db)[3],
+                                                    const OtfConst &o, float2 (&cf)[Q + 2])
 {
-  double dr[3];
-#pragma unroll
-  for(int k = 0; k < 3; ++k) dr[k] = pobs[k] - psrc[k];
-  const double sq = (dr[0] * dr[0] + dr[1] * dr[1]) + dr[2] * dr[2];
-  const double nrm = sqrt(sq);
-  double idelay;
-  const double xd = modf(nrm / (p.c0 * p.dt), &idelay);
-  const int fd = (int)idelay;
-
-  const float x = (float)xd;
-  const float inv_dt = (float)(1.0 / p.dt);
-  float w0[Q + 1], w1[Q + 1], w2[Q + 1];
-#pragma unroll
-  for(int b = 0; b <= Q; ++b) {
-    float e[Q + 1];
-    e[0] = 1.f;
-#pragma unroll
-    for(int k = 1; k <= Q; ++k) e[k] = 0.f;
-    int n = 0;
-#pragma unroll
-    for(int m = 0; m <= Q; ++m) {
-      if(m == b) continue;
-      const float f = x - (float)m;
-      ++n;
-#pragma unroll
-      for(int k = Q; k >= 1; --k)
-        if(k <= n) e[k] = fmaf(f, e[k - 1], e[k]);
-    }
-    float den = 1.f;
-#pragma unroll
-    for(int m = 0; m <= Q; ++m)
-      if(m != b) den *= (float)(b - m);  // an exact integer (|den| <= 7!)
-    const float id = 1.f / den;
-    w0[b] = e[Q] * id;
-    w1[b] = -(e[Q - 1] * id) * inv_dt;
-    w2[b] = Q >= 2 ? (2.f * (e[Q >= 2 ? Q - 2 : 0] * id)) * (inv_dt * inv_dt) : 0.f;
-  }
-
-  const float drf[3] = {(float)dr[0], (float)dr[1], (float)dr[2]};
-  const float df_s[3] = {(float)dsrc[0], (float)dsrc[1], (float)dsrc[2]};
-  const float df_o[3] = {(float)dobs[0], (float)dobs[1], (float)dobs[2]};
-  const float dd = fmaf(df_o[2], df_s[2], fmaf(df_o[1], df_s[1], df_o[0] * df_s[0]));
-  const float ar = fmaf(df_o[2], drf[2], fmaf(df_o[1], drf[1], df_o[0] * drf[0]));
-  const float br = fmaf(df_s[2], drf[2], fmaf(df_s[1], drf[1], df_s[0] * drf[0]));
-  const float inv_r = (float)(1.0 / nrm), inv_sq = inv_r * inv_r;
+  const float x = (float)g.x;
+  const float drf[3] = {(float)g.dr[0], (float)g.dr[1], (float)g.dr[2]};
+  const float fa[3] = {(float)da[0], (float)da[1], (float)da[2]};
+  const float fb[3] = {(float)db[0], (float)db[1], (float)db[2]};
+  const float dd = fmaf(fa[2], fb[2], fmaf(fa[1], fb[1], fa[0] * fb[0]));
+  const float ar = fmaf(fa[2], drf[2], fmaf(fa[1], drf[1], fa[0] * drf[0]));
+  const float br = fmaf(fb[2], drf[2], fmaf(fb[1], drf[1], fb[0] * drf[0]));
+  const float inv_r = (float)rcp_newton(g.nrm), inv_sq = inv_r * inv_r;
   const float ab = (ar * br) * inv_sq;
   const float g3 = fmaf(-3.f, ab, dd), g1 = dd - ab;
-  const float c0 = (float)p.c0;
-  const float G0 = (g3 * (c0 * c0)) * (inv_sq * inv_r);
-  const float G1 = (g3 * c0) * inv_sq;
+  const float G0 = (g3 * (float)o.c0_sq) * (inv_sq * inv_r);
+  const float G1 = (g3 * (float)o.c0) * inv_sq;
   const float G2 = g1 * inv_r;
-  const float A = (float)(p.mu0 / (4 * M_PI * p.hbar));
-  if(p.frame == 0) {
-    const double om = p.omega;
-    const double ph = (-om * nrm) / p.c0;
-    const double red = ph - 6.283185307179586 * rint(ph * 0.15915494309189535);
-    float sn, cs;
-    sincosf((float)red, &sn, &cs);
-    const float2 sc = make_float2(-A * cs, -A * sn);
-    const float omf = (float)om, om2 = omf * omf;
-#pragma unroll
-    for(int i = 0; i <= Q; ++i) {
-      const float re = fmaf(G2, fmaf(-om2, w0[i], w2[i]), fmaf(G0, w0[i], G1 * w1[i]));
-      const float im = omf * fmaf(G1, w0[i], 2.f * (G2 * w1[i]));
-      cf[i] = make_float2(fmaf(sc.x, re, -sc.y * im), fmaf(sc.x, im, sc.y * re));
-    }
-    const float rs = fmaf(-om2, G2, G0), is = omf * G1;
-    cf[Q + 1] = make_float2(fmaf(sc.x, rs, -sc.y * is), fmaf(sc.x, is, sc.y * rs));
+  const float A = (float)o.A, idt = (float)o.inv_dt, idt2 = (float)(2.0 * o.inv_dt2);
+  if(LAB) {
+    const float al = A * G0, be = -(A * G1) * idt, ga = (A * G2) * idt2;
+    lagrange_jets<Q>(x, [&](int b, const Jet<float> &j) {
+      cf[b] = make_float2((float)node_scale<Q>(b) * fmaf(ga, j.h, fmaf(be, j.d, al * j.v)), 0.f);
+    });
+    cf[Q + 1] = make_float2(al, 0.f);
   } else {
-#pragma unroll
-    for(int i = 0; i <= Q; ++i) cf[i] = make_float2(A * fmaf(G2, w2[i], fmaf(G0, w0[i], G1 * w1[i])), 0.f);
-    cf[Q + 1] = make_float2(A * G0, 0.f);
+    const double ph = g.nrm * o.half_turns;
+    float sn, cs;
+    sincospif((float)fma(-2.0, rint(0.5 * ph), ph), &sn, &cs);
+    const float sx = -(A * cs), sy = A * sn;
+    const float om = (float)o.om;
+    const float ar0 = fmaf(-(float)o.om_sq, G2, G0), ai0 = om * G1;
+    const float br0 = -G1 * idt, bi0 = -2.f * (om * G2) * idt;
+    const float gr0 = G2 * idt2;
+    const float alx = fmaf(sx, ar0, -(sy * ai0)), aly = fmaf(sx, ai0, sy * ar0);
+    const float bex = fmaf(sx, br0, -(sy * bi0)), bey = fmaf(sx, bi0, sy * br0);
+    const float gax = sx * gr0, gay = sy * gr0;
+    lagrange_jets<Q>(x, [&](int b, const Jet<float> &j) {
+      const float id = (float)node_scale<Q>(b);
+      cf[b] = make_float2(id * fmaf(gax, j.h, fmaf(bex, j.d, alx * j.v)), id * fmaf(gay, j.h, fmaf(bey, j.d, aly * j.v)));
+    });
+    cf[Q + 1] = make_float2(alx, aly);
   }
-  if(xd == 0.0) {
-    // the reference's weights at x = 0: node 0's are finite, every other
-    // node's w1 and w2 are 0 * inf = NaN (lagrange_set.cpp:25-33); the sum
-    // carries them
+  if(g.x == 0.0) {
 #pragma unroll
     for(int i = 1; i <= Q + 1; ++i) cf[i] = make_float2(__int_as_float(0x7fc00000), 0.f);
   }
-  return fd;
 }
 
 }  // namespace qg

@@ -20,7 +20,8 @@ constexpr int kTimeBlock = 16;   // K: steps per pass of the far-pair kernel
 constexpr int kRingMirror = 24;  // slots mirrored past the ring end (>= K+q)
 constexpr int kTile = 32;        // dots per table tile (a warp's 32 targets)
 constexpr int kTilePairs = kTile * kTile;
-constexpr int kTileGroup = 4;    // source tiles one warp sums before writing
+constexpr int kTileGroup = 4;    // source tiles per group of the far kernel
+constexpr int kFarWarps = 4;     // warps (tasks) per far-kernel block
 constexpr int kPcDepth = 23;     // PC ring: 22 past steps + the current one
 constexpr int kStepBlock = 128;  // threads per block of the dot-step kernel
 constexpr int kBadNone = 0x7fffffff;
@@ -38,6 +39,14 @@ struct CoefParams {
   double c0, dt, mu0, hbar, omega;
   int q;
   int frame;
+};
+
+// The same constants as the on-the-fly kernels use them.
+struct OtfConst {
+  double c0dt, inv_c0dt;  // c0 dt and its correctly rounded reciprocal
+  double c0, c0_sq, A;    // A = mu0 / (4 pi hbar)
+  double inv_dt, inv_dt2;
+  double om, om_sq, half_turns;  // half_turns = omega / (pi c0)
 };
 
 struct PulseParams {
@@ -64,8 +73,21 @@ struct TableArgs {
   CoefParams cp;
 };
 
+// What a far launch knows of its windows.  kFormAny: nothing; samples before
+// step -22 are skipped.  kFormPlain: no sample needs to be: every window starts
+// at step -22 or later (blocks past the largest delay), or every coefficient
+// is finite and the ring slots of steps before -22 still hold the zeros they
+// were reset to (the history was only ever written by the run itself), whose
+// products are +-0 and leave an accumulator that started at +0 bit for bit
+// as it was.  Both forms give the same bits.  The plain form serves the first
+// blocks too: testing or zeroing the dead samples there made a 640-step run
+// of 4096 dots 2-4 % slower than it began, and the tests' registers cost the
+// steady state as well (641 against 784 us a launch, zeroing).
+enum : int { kFormAny = 0, kFormPlain = 1 };
+
 // Arguments of the far-pair kernel: K steps of the pair sum for every pair
-// with floor delay >= K, from one pass over the table.
+// with floor delay >= K, from one pass over the table (or one evaluation of
+// the coefficients).
 struct FarArgs {
   const int *delay;     // [nT][nT][kTilePairs] ordered tile pairs
   const double2 *coef;  // [nT][nT][q+1][kTilePairs]
@@ -76,35 +98,42 @@ struct FarArgs {
   const float2 *ring32w;
   const float2 *ring32d;
   int mixed;
-  double2 *partial;     // [K][nG][n_pad] per source-tile group
+  double2 *partial;     // [K][nP][n_pad] per source part
   double2 *field;       // [K][n_pad] far-pair field
-  unsigned *tile_done;  // [nT] completion counters (zero between launches)
-  int n_pad, nT, nG, W, stride, q, frame;
+  int n_pad, nT, W, stride, q, frame;
+  // sources: groups of `group` source tiles, each cut into `parts` parts of
+  // `unit` sources (the last of a group may be shorter or empty); nP parts in
+  // all.  A part's sum is one partial; the partials are added in part order.
+  int group, parts, unit, nP;
   const int *d_t0;      // first step of the block
   int *far_t0_out;      // receives *d_t0 (read by the dot-step kernels)
-  int variant;          // kernel variant (same results), see qg_far.cu
-  // task order: 0 target-tile major (a block's warps take consecutive source
-  // groups of one target tile), 1 source-group major (they take one source
-  // group of consecutive target tiles, so they read the same history rows);
-  // the same sums either way
-  int gmajor;
-  int *d_bad;           // a far-kernel wait that ran out sets it to -3
-  // 1: some windows may start before step -22 (the first blocks of a run)
-  // and every far pair's coefficients are finite; the FP64 table launch then
-  // takes the first-blocks form whatever the variant (same results)
-  int early;
-  // on-the-fly coefficients (no table): dot data, constants, and the source
-  // tiles per warp (nG = ceil(nT / group) groups)
+  int form;             // what is known of the launch's windows: kFormAny or kFormPlain
+  // on-the-fly coefficients (no table): dot data and constants
   int otf;
-  int group;
   const double *pos;    // [n_pad][3]
   const double *dip;    // [n_pad][3]
   const int *user;      // internal -> user index, -1 for padding
-  CoefParams cp;
+  OtfConst oc;
   // target tiles [tile_lo, tile_lo + tile_n) only (a shard of a sharded
   // handle; on-the-fly kernel); tile_n == 0: all nT
   int tile_lo, tile_n;
 };
+
+// Parts per source group (FarArgs::parts).  A far task, one warp's, is a
+// target tile x one part, and 148 SMs hold 1776 at once (3 blocks of 4 warps).
+// While there are fewer, a launch lasts one task, so the groups are cut until
+// the tasks fill the device, or a part has 8 sources (beginning and ending a
+// task cost about as much as 4).  The cut fixes the association of the far
+// sums, so it depends on the ensemble and the group alone: the same alone, in
+// a batch and in a shard.
+inline int far_parts(int nT, int group)
+{
+  const long long tasks = (long long)nT * ((nT + group - 1) / group);
+  const int n = group * kTile;
+  int parts = 1;
+  while(tasks * (parts + 1) <= 1776 && n / (parts + 1) >= 8) ++parts;
+  return parts;
+}
 
 // Arguments of the per-dot step kernels.
 struct StepArgs {
@@ -175,20 +204,19 @@ constexpr int kNoAllocMaxDots = 4096;
 constexpr int kNoAllocMaxTiles = kNoAllocMaxDots / kTile;
 constexpr int kNoAllocMaxGroups = (kNoAllocMaxTiles + kTileGroup - 1) / kTileGroup;
 constexpr size_t kNoAllocScratchTotal = 16ull * kNoAllocMaxGroups * kNoAllocMaxDots + 16ull * kNoAllocMaxDots +
-                                        256 * ((4ull * kNoAllocMaxTiles + 255) / 256) + 256;
+                                        256;
 struct NoAllocScratch {
   double2 *partial;    // [kNoAllocMaxGroups][n_pad]
   double2 *field;      // [n_pad]
-  unsigned *tile_done; // [nT]
   int *ints;           // [0] step, [1] far_t0 written by the kernel
-  size_t tile_bytes;
 };
 qg_status noalloc_scratch(NoAllocScratch *out);
+// The far field of one step (slice 0 of the field): evaluations
 void launch_far_step1(const FarArgs &a, void *stream);
-// mixed: 0 FP64 members, 1 mixed (scalar FP32 convolution), 2 mixed (packed
-// FP32 pairs; the same bits as 1)
-void launch_far_batch(const FarArgs *args, const int *task_off, int n_ens, int q, int frame, int mixed,
-                      int grid, void *stream);
+// Many ensembles: block_off[e] = first far block of ensemble e (far_blocks of
+// each), tile_off[e] = its first 32-dot tile; totals at [n_ens]
+void launch_far_batch(const FarArgs *args, const int *block_off, const int *tile_off, int n_ens, int blocks, int tiles,
+                      int q, int frame, int mixed, int form, void *stream);
 void launch_ring32_rebuild(const StepArgs &a, void *stream);
 // Sharded handles: a shard's rho01 at step t for internal dots [lo, hi)
 // into out[0 .. hi-lo), and the other dots' rho01 at step t from the full
@@ -206,11 +234,20 @@ int step_block_max_blocks(int q, int mid_cache, int hist_cap);
 void launch_step_batch(const StepArgs *args, const int *block_off, int n_ens, int total_blocks, int n_time,
                        int k, bool pipe, void *stream);
 
+// Far-kernel tasks (warps) of one ensemble, and the blocks that hold them.
+__host__ __device__ inline int far_tasks(const FarArgs &a) { return (a.tile_n > 0 ? a.tile_n : a.nT) * a.nP; }
+inline int far_blocks(const FarArgs &a) { return (far_tasks(a) + kFarWarps - 1) / kFarWarps; }
+
 // Launchers (defined in the .cu files).
 void launch_table_build(const TableArgs &a, int q, void *stream);
 void launch_far(const FarArgs &a, void *stream);
 void launch_far_otf(const FarArgs &a, void *stream);
-void launch_max_delay(const double *pos, const int *user, int n_pad, double c0dt, int *max_delay, void *stream);
+void launch_far_otf_step1(const FarArgs &a, void *stream);
+// field[k][.] = the sum of the partials over the parts, in part order, for k < steps
+void launch_far_reduce(const FarArgs &a, int steps, void *stream);
+// whole: += far pairs at a whole delay (fraction 0)
+void launch_max_delay(const double *pos, const int *user, int n_pad, double c0dt, int *max_delay,
+                      unsigned long long *whole, void *stream);
 void launch_near_find(const double *pos, const int *user, int n_pad, double c0dt, int below, int *out_pairs,
                       unsigned long long *counter, unsigned long long cap, void *stream);
 void launch_pair_list_coef(const TableArgs &a, int q, const int *pairs, long long m, double2 *out, void *stream);

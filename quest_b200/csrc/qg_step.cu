@@ -47,21 +47,6 @@ __device__ __forceinline__ double2 prefactor(double2 r, int frame)
   return frame == 0 ? r : make_double2(2 * r.x, 0.0);
 }
 
-// x / t given y = 1/t correctly rounded: q0 = x*y, the remainder x - q0*t
-// exact in one fused multiply-add, then q0 + r*y rounded once.  This is
-// Markstein's correction step (P. W. Markstein, IBM J. Res. Develop. 34(1),
-// 1990): with y within half an ulp of 1/t and q0 within one ulp of x/t it
-// returns the correctly rounded quotient, i.e. exactly x / t, barring
-// underflow and overflow.  r == 0 means q0 is exact (and keeps the sign of a
-// zero quotient).  Four independent divisions per evaluation become twelve
-// independent flops instead of four serial division sequences.
-__device__ __forceinline__ double div_by(double x, double t, double y)
-{
-  const double q0 = x * y;
-  const double r = fma(-q0, t, x);
-  return r == 0.0 ? q0 : fma(r, y, q0);
-}
-
 // Per-dot constants of the right-hand side.
 struct DotConst {
   double det, t1, t2, inv1, inv2;

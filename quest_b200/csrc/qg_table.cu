@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(128) table_build_kernel(TableArgs a)
   if(fd < kTimeBlock) atomicAdd(a.near_count + 1, 1ULL);
   if(fd >= kTimeBlock) {
     // far pairs with a non-finite coefficient (an integer delay): the far
-    // kernels' first-blocks form is not used for such a table
+    // kernels' plain form is not used for the first blocks of such a table
     bool fin = true;
 #pragma unroll
     for(int i = 0; i <= Q; ++i) fin = fin && isfinite(coef[i].x) && isfinite(coef[i].y);
@@ -172,9 +172,10 @@ __global__ void near_find_kernel(const double *pos, const int *user, int n_pad, 
 }
 
 // The largest floor delay over all pairs (for the ring depth when no table
-// is built), with the delay arithmetic of pair_coef_ref.
+// is built), with the delay arithmetic of pair_coef_ref, and the far pairs at
+// a whole delay, whose Lagrange weights are not finite.
 __global__ void __launch_bounds__(256) max_delay_kernel(const double *pos, const int *user, int n_pad, double c0dt,
-                                                        int *out)
+                                                        int *out, unsigned long long *whole)
 {
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nt = (n_pad + kTile - 1) / kTile;
@@ -194,20 +195,22 @@ __global__ void __launch_bounds__(256) max_delay_kernel(const double *pos, const
       for(int k = 0; k < 3; ++k) dr[k] = pos[3 * io + k] - pos[3 * is + k];
       const double nrm = sqrt((dr[0] * dr[0] + dr[1] * dr[1]) + dr[2] * dr[2]);
       double idelay;
-      modf(nrm / c0dt, &idelay);
+      const double frac = modf(nrm / c0dt, &idelay);
       v = (int)idelay;
+      if(v >= kTimeBlock && frac == 0.0) atomicAdd(whole, 1ULL);
     }
   }
   v = __reduce_max_sync(0xffffffffu, v);
   if((threadIdx.x & 31) == 0 && v >= 0) atomicMax(out, v);
 }
 
-void launch_max_delay(const double *pos, const int *user, int n_pad, double c0dt, int *max_delay, void *stream)
+void launch_max_delay(const double *pos, const int *user, int n_pad, double c0dt, int *max_delay,
+                      unsigned long long *whole, void *stream)
 {
   const long long nt = (n_pad + kTile - 1) / kTile;
   const long long total = nt * (nt + 1) / 2 * kTilePairs;
   const unsigned blocks = (unsigned)((total + 255) / 256);
-  max_delay_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(pos, user, n_pad, c0dt, max_delay);
+  max_delay_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(pos, user, n_pad, c0dt, max_delay, whole);
 }
 
 // FP64 coefficients of listed pairs (the per-step mid list), computed as the
