@@ -94,6 +94,7 @@ struct qg_handle_s {
 
   bool fused = true;
   int step_blocks = 0;
+  GroupShape group_launch{};  // the general form's launch (not fused)
   // all 16 steps of a block in one cooperative launch (fused form, every
   // 32-dot block resident at once); otherwise one launch per step
   bool block_step = false, block_step_ok = false;
@@ -698,6 +699,7 @@ static qg_status build_lists(qg_handle *h, const TableArgs &ta)
     }
   }
   h->block_step = h->block_step_ok;
+  if(!h->fused) h->group_launch = group_shape(h->n_pad, gptr.data());
 
   auto upload_i = [&](int **dst, const std::vector<int> &v) -> qg_status {
     QG_TRY(dalloc(h, dst, v.size()));
@@ -1042,7 +1044,7 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
   h->max_parts = max_parts(h->nT, h->group, h->otf);
   QG_TRY(dalloc(h, &h->d_partial, (size_t)kTimeBlock * h->max_parts * h->n_pad));
   QG_TRY(dalloc(h, &h->d_field, (size_t)kTimeBlock * h->n_pad));
-  QG_TRY(dalloc(h, &h->d_scratch, (size_t)h->n_pad * 8));
+  QG_TRY(dalloc(h, &h->d_scratch, (size_t)h->n_pad * kScratchPerDot));
   h->traj_k = traj_steps(n);
   QG_TRY(dalloc(h, &h->d_traj, (size_t)2 * h->traj_k * n * 2));
   QG_TRY(dalloc(h, &h->d_io, (size_t)n));
@@ -1276,23 +1278,25 @@ static void enqueue_far(qg_handle *h, int t0, bool at_boundary, cudaEvent_t ea, 
   if(eb) record_event(h, eb);
 }
 
-// Steps k0 .. k1-1 of the current block in one cooperative launch.
+// Steps k0 .. k1-1 of the current block in one launch.
 static void enqueue_step_block(qg_handle *h, int k0, int k1, bool traj)
 {
-  StepArgs a = h->step_args(false);
+  StepArgs a = h->step_args(!h->fused);
   if(traj) a.traj = h->d_traj;
-  launch_step_block(a, k0, k1, h->step_blocks, h->d_flags, h->stream);
+  if(h->fused)
+    launch_step_block(a, k0, k1, h->step_blocks, h->d_flags, h->stream);
+  else
+    launch_step_group(a, k0, k1, h->group_launch, h->d_flags, h->stream);
 }
 
 static void enqueue_dot_step(qg_handle *h, int k, bool traj)
 {
   StepArgs a = h->step_args(!h->fused);
   if(traj) a.traj = h->d_traj;
-  if(h->fused) {
+  if(h->fused)
     launch_step_fused(a, k, h->shard_world > 1 ? h->blk_hi - h->blk_lo : h->step_blocks, h->stream);
-  } else {
-    for(int ph = 0; ph <= kCorrectorSteps + 1; ++ph) launch_step_general(a, k, ph, h->stream);
-  }
+  else
+    launch_step_group(a, k, k + 1, h->group_launch, h->d_flags, h->stream);
 }
 
 // One K-step block starting on a boundary: far kernel + K dot steps
@@ -1304,7 +1308,7 @@ static qg_status capture_block(qg_handle *h, int gi, int prof, cudaGraphExec_t *
   QG_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   enqueue_far(h, 0, true, prof >= 0 ? h->pev[prof][0] : nullptr, prof >= 0 ? h->pev[prof][1] : nullptr,
               gi / 2);
-  if(h->block_step)
+  if(h->block_step || !h->fused)
     enqueue_step_block(h, 0, kTimeBlock, traj != 0);
   else
     for(int k = 0; k < kTimeBlock; ++k) enqueue_dot_step(h, k, traj != 0);
@@ -1331,7 +1335,7 @@ static qg_status collect_prof(qg_handle *h, int i)
   h->pair_ms += far;
   h->pair_launches += 1;
   h->step_ms += steps;
-  h->step_launches += h->block_step ? 1 : kTimeBlock * (h->fused ? 1 : kCorrectorSteps + 2);
+  h->step_launches += h->block_step || !h->fused ? 1 : kTimeBlock;
   h->pending[i] = false;
   return QG_OK;
 }
@@ -1388,7 +1392,7 @@ static qg_status collect_events(qg_handle *h, int nev, int nstep)
       cudaEventElapsedTime(&ms, h->ev_c[j], h->ev_d[j]);
       h->step_ms += ms;
     }
-    h->step_launches += h->fused ? nstep : nstep * (kCorrectorSteps + 2);
+    h->step_launches += nstep;
   }
   return QG_OK;
 }
@@ -1420,7 +1424,7 @@ static qg_status launch_steps(qg_handle *h, int t, int count, bool traj)
       h->far_block = t0;
     }
     // the rest of this block (or of the run) in one launch when allowed
-    const int span = h->block_step ? std::min(count, t0 + kTimeBlock - t) : 1;
+    const int span = h->block_step || !h->fused ? std::min(count, t0 + kTimeBlock - t) : 1;
     if(h->profile) cudaEventRecord(h->ev_c[nstep], h->stream);
     if(span > 1)
       enqueue_step_block(h, t - t0, t - t0 + span, traj);
@@ -1615,7 +1619,7 @@ extern "C" qg_status qg_run(qg_handle *h, int n_steps, double *rho_out, int *bad
   QG_CUDA(cudaGetLastError());
   h->next_step = t_start + n_steps;
   if(bad == -2)
-    return qg_fail(QG_ERR_CUDA, "qg_run: a wait in the step-block kernel timed out");
+    return qg_fail(QG_ERR_CUDA, "qg_run: a wait in the step kernel timed out");
   if(bad < 0)
     return qg_fail(QG_ERR_CUDA, "qg_run: internal scheduling error (far block or trajectory row)");
   if(bad != kBadNone) {
@@ -2364,7 +2368,7 @@ extern "C" qg_status qg_footprint(int n, const qg_params *p, double side, size_t
   b += sizeof(double2) * (size_t)n_pad * (W + kRingMirror) * (mixed ? 2 : 1);
   b += sizeof(double2) * (size_t)kPcDepth * 4 * n_pad;
   b += sizeof(double2) * (size_t)kTimeBlock * (max_parts(nT, group, otf) + 1) * n_pad;
-  b += sizeof(double2) * (size_t)n_pad * 8;
+  b += sizeof(double2) * (size_t)n_pad * kScratchPerDot;
   b += sizeof(double) * (size_t)n_pad * 9 + sizeof(int) * (size_t)n_pad * 2;
   const long long K = traj_steps(n);
   b += sizeof(double2) * (size_t)(2 * K * n * 2) + sizeof(double2) * (size_t)n;  // trajectory + io staging

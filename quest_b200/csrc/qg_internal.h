@@ -23,7 +23,6 @@ constexpr int kTilePairs = kTile * kTile;
 constexpr int kTileGroup = 4;    // source tiles per group of the far kernel
 constexpr int kFarWarps = 4;     // warps (tasks) per far-kernel block
 constexpr int kPcDepth = 23;     // PC ring: 22 past steps + the current one
-constexpr int kStepBlock = 128;  // threads per block of the dot-step kernel
 constexpr int kBadNone = 0x7fffffff;
 
 // Weights as passed to kernels (copy of qg_weights).
@@ -135,6 +134,11 @@ inline int far_parts(int nT, int group)
   return parts;
 }
 
+// A dot's state in the general step form (RowState, qg_step.cu), and the
+// double2 per dot of StepArgs::scratch.
+constexpr int kRowStateBytes = 160;
+constexpr int kScratchPerDot = 2 + kRowStateBytes / 16;
+
 // Arguments of the per-dot step kernels.
 struct StepArgs {
   int n, n_pad, nT, W, stride, q, frame;
@@ -181,8 +185,7 @@ struct StepArgs {
   const int *near_ptr;
   const int *near_idx;
   const double2 *near_coef;
-  // general path scratch
-  double2 *scratch;      // [n_pad][8]: past field, pulse, H (2 complex), cur rho x2
+    double2 *scratch;      // general form: [2][n_pad] iterates exchanged by its grid, then kRowStateBytes a dot
   double2 *traj;         // [k][n][2] user order or null
   int traj_rows;         // rows allocated in traj
   const int *traj_t0;
@@ -229,6 +232,15 @@ void launch_gather_bad(const StepArgs *args, int n, int *out, void *stream);
 // the polls on one block's count do not queue behind those on another's).
 constexpr int kFlagStride = 32;
 void launch_step_block(const StepArgs &a, int k0, int k1, int nblocks, unsigned *flags, void *stream);
+// The general step form's launch: one cluster or a cooperative grid of
+// `blocks` blocks of `rows` dots, `cache` near entries in shared memory,
+// stage: the iterates copied there, state: the rows' states kept there
+struct GroupShape {
+  int cluster, blocks, rows, cache, stage, state;
+  size_t smem;
+};
+GroupShape group_shape(int n_pad, const int *near_ptr);
+void launch_step_group(const StepArgs &a, int k0, int k1, const GroupShape &g, unsigned *counter, void *stream);
 int step_block_max_blocks(int q, int mid_cache, int hist_cap);
 // pipe: the mid list staged with several entries' loads in flight (same sums)
 void launch_step_batch(const StepArgs *args, const int *block_off, int n_ens, int total_blocks, int n_time,
@@ -255,7 +267,6 @@ void launch_pair_list_coef(const TableArgs &a, int q, const int *pairs, long lon
 void launch_gather_rows(const double2 *src, const long long *rows, int width, long long n, double2 *dst,
                         void *stream);
 void launch_step_fused(const StepArgs &a, int k, int nblocks, void *stream);
-void launch_step_general(const StepArgs &a, int k, int phase, void *stream);
 void launch_eval_field(const StepArgs &a, const int *d_eval_step, double2 *out_user, void *stream);
 void launch_pulse_field(const StepArgs &a, int step, double2 *out_user, void *stream);
 void launch_set_int(int *p, int v, void *stream);

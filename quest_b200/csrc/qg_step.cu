@@ -17,12 +17,12 @@
 // stop after a non-finite value: the first such step is recorded and every
 // step is computed, so the cost per step does not depend on the data.
 //
-// Two forms.  The fused kernel runs predictor, 11 evaluations and 10
-// corrections in one launch: every connected group of dots coupled at delay
-// 0 is placed inside one thread block, so a __syncthreads between
-// iterations is the only synchronisation needed.  The general form (used when
-// such a group is larger than a block, e.g. when c0*dt exceeds the dot
-// spacing and every pair has delay 0) runs one launch per evaluation.
+// Two forms.  The fused kernels run predictor, 11 evaluations and 10
+// corrections of a step with block-wide synchronisation alone: every connected
+// group of dots coupled at delay 0 is placed inside one 32-dot thread block.
+// The general form (used when such a group is larger, e.g. when c0*dt exceeds
+// the dot spacing and every pair has delay 0) exchanges the iterates between
+// all its blocks after every correction.
 //
 // Per-dot state in HBM:
 //   pcr[slot][k][dot]   k = rho00, rho01, drho00, drho01 for the last 23
@@ -105,34 +105,6 @@ __device__ __forceinline__ double pulse_rabi(const StepArgs &a, int idx, int t)
 {
   const double *d = a.dip + 3 * idx;
   return pulse_at(a, pulse_kr(a, idx), d[0], d[1], d[2], t);
-}
-
-// Predictor value P and corrector base H (the history part of the
-// corrector sum) from the n_time-step window (NT > 0: compile-time width,
-// loop unrolled so the window's loads are all in flight together).
-template <int NT>
-__device__ __forceinline__ void pc_window(const StepArgs &a, int idx, int t, double2 (&P)[2],
-                                          double2 (&H)[2])
-{
-  P[0] = P[1] = H[0] = H[1] = make_double2(0.0, 0.0);
-  const int nt = NT > 0 ? NT : a.w.n_time;
-  const double dt = a.dt;
-#pragma unroll
-  for(int h = 0; h < (NT > 0 ? NT : a.w.n_time); ++h) {
-    const int s = pc_slot(t - nt + h);
-    const double2 *base = a.pcr + (long long)s * 4 * a.n_pad + idx;
-    const double2 x0 = base[0], x1 = base[a.n_pad], y0 = base[2 * a.n_pad], y1 = base[3 * a.n_pad];
-    const double p0 = a.w.ps[h], p1 = a.w.ps[nt + h];
-    const double c0 = a.w.cs[h], c1 = a.w.cs[nt + h];
-    P[0].x += x0.x * p0 + (y0.x * p1) * dt;
-    P[0].y += x0.y * p0 + (y0.y * p1) * dt;
-    P[1].x += x1.x * p0 + (y1.x * p1) * dt;
-    P[1].y += x1.y * p0 + (y1.y * p1) * dt;
-    H[0].x += x0.x * c0 + (y0.x * c1) * dt;
-    H[0].y += x0.y * c0 + (y0.y * c1) * dt;
-    H[1].x += x1.x * c0 + (y1.x * c1) * dt;
-    H[1].y += x1.y * c0 + (y1.y * c1) * dt;
-  }
 }
 
 __device__ __forceinline__ int ring_slot(int t, int W) { return ((t % W) + W) % W; }
@@ -1072,58 +1044,376 @@ int step_block_max_blocks(int q, int mid_cache, int hist_cap)
   return sms * per;
 }
 
-// General form, one launch per phase: phase 0 predicts, phases 1..11 are the
-// 11 evaluations (each followed by a correction except the last).
-// scratch[idx*8 + k]: 0 past field, 1 pulse, 2-3 H, 4-5 rho (even
-// iterations), 6-7 rho (odd iterations).
-__global__ void __launch_bounds__(kStepBlock) step_general_kernel(StepArgs a, int k, int phase)
+// ---- groups coupled at delay 0 that exceed a block -----------------------------
+// The general form: the steps k0 .. k1-1 of a block in one launch, a warp per
+// dot for its sums and a thread per dot for its state, the iterates exchanged
+// between all blocks after every correction (11 times a step).  Each thread block keeps its dots' part of the near list in
+// shared memory for the launch (when it fits), and all dots' iterates twice
+// (the exchange's two turns).
+//
+// What bounds it is the exchange: 11 dependent evaluations per step, each a
+// dense sum over the group.  Up to kClusterBlocks blocks (256 dots) run as one
+// thread-block cluster, whose blocks write their iterates into each other's
+// shared memory and meet at the hardware's cluster barrier; larger ensembles
+// run as a cooperative grid that exchanges through L2 and meets at a
+// counter in global memory (a wait that runs out sets *a.d_bad to -2).  One
+// launch per evaluation with a thread per dot, the form this replaces, took
+// 807 us a step at 256 dots.
+constexpr int kGroupWarps = 16;
+constexpr int kGroupThreads = 32 * kGroupWarps;
+constexpr int kClusterBlocks = 16;
+constexpr int kNearFlight = 4;
+constexpr int kGridSpins = 1 << 20;  // polls of a grid wait, x ~0.7 us: about a second
+
+// A row's state between iterations, in shared memory as far as it fits.
+struct RowState {
+  double2 r[2], H[2], past, near;
+  double pul;
+  DotConst dc;
+  int live, e0, e1, pad;  // live; its near entries [e0, e1)
+};
+static_assert(sizeof(RowState) == kRowStateBytes, "scratch size");
+
+__device__ __forceinline__ double2 warp_sum(double2 v)
 {
-  const int idx = blockIdx.x * kStepBlock + threadIdx.x;
-  const int t = *a.far_t0 + k;
-  const bool live = idx < a.n_pad && a.user[idx] >= 0;
-  double2 *sc = a.scratch + (long long)idx * 8;
-  if(phase == 0) {
-    if(live) {
-      double2 P[2], H[2];
-      if(a.w.n_time == 22)
-        pc_window<22>(a, idx, t, P, H);
-      else
-        pc_window<0>(a, idx, t, P, H);
-      sc[0] = past_field(a, idx, t, k);
-      sc[1] = make_double2(pulse_rabi(a, idx, t), 0.0);
-      sc[2] = H[0];
-      sc[3] = H[1];
-      sc[4] = P[0];
-      sc[5] = P[1];
-    }
-    return;
+#pragma unroll
+  for(int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
   }
-  const int it = phase - 1;
-  const int rd = (it & 1) ? 6 : 4, wr = (it & 1) ? 4 : 6;
-  if(live) {
-    double2 r[2] = {sc[rd], sc[rd + 1]};
-    double2 nf = make_double2(0.0, 0.0);
-    for(int e = a.near_ptr[idx]; e < a.near_ptr[idx + 1]; ++e) {
-      const int b = a.near_idx[e];
-      const double2 v = cmul(prefactor(a.scratch[(long long)b * 8 + rd + 1], a.frame), a.near_coef[e]);
-      nf.x += v.x;
-      nf.y += v.y;
+  return v;
+}
+
+// Field of a dot at step t from every tap that reads an earlier step, without
+// the far part: a warp's lanes over the (entry, tap) products of its mid list,
+// kPastFlight at a time, so that their coefficients are read in one run and
+// their history samples together.
+constexpr int kPastFlight = 8;
+
+__device__ __forceinline__ double2 group_past(const StepArgs &a, int idx, int t)
+{
+  const int q1 = a.q + 1, lane = threadIdx.x & 31, tslot = ring_slot(t, a.W);
+  const int m0 = a.mid_ptr[idx] * q1, m1 = a.mid_ptr[idx + 1] * q1;
+  double2 f[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+  for(int j0 = m0 + lane; j0 < m1; j0 += 32 * kPastFlight) {
+    // no branch between the loads: a product past the end repeats the last
+    // one, and is not added
+    int e[kPastFlight], d[kPastFlight], b[kPastFlight];
+    double2 v[kPastFlight], c[kPastFlight];
+#pragma unroll
+    for(int u = 0; u < kPastFlight; ++u) {
+      e[u] = min(j0 + 32 * u, m1 - 1) / q1;
+      d[u] = __ldg(a.mid_delay + e[u]);
+      b[u] = __ldg(a.mid_idx + e[u]);
     }
-    const double2 past = sc[0];
-    const double pul = sc[1].x;
-    const double2 om = make_double2((0.0 + pul) + (past.x + nf.x), 0.0 + (past.y + nf.y));
-    double2 dr[2];
-    liouville(r[0], r[1], om, dot_const(a, idx, true), dr[0], dr[1]);
-    if(it < kCorrectorSteps) {
-      const double2 H[2] = {sc[2], sc[3]};
-      corrector(a, dr, H, r);
-      sc[wr] = r[0];
-      sc[wr + 1] = r[1];
-    } else {
-      finish_dot(a, idx, t, r, dr);
+#pragma unroll
+    for(int u = 0; u < kPastFlight; ++u) {
+      const int j = min(j0 + 32 * u, m1 - 1), back = d[u] + (j - e[u] * q1);
+      const int slot = tslot - back + (tslot < back ? a.W : 0);
+      v[u] = __ldcg(a.ring + (long long)b[u] * a.stride + slot);
+      c[u] = __ldg(a.mid_coef + j);
+    }
+#pragma unroll
+    for(int u = 0; u < kPastFlight; ++u) {
+      const int j = j0 + 32 * u, back = d[u] + (j - e[u] * q1);
+      if(j < m1 && t - back >= -kWindow && back >= 1) {
+        const double2 p = cmul(prefactor(v[u], a.frame), c[u]);
+        f[u & 1].x += p.x;
+        f[u & 1].y += p.y;
+      }
     }
   }
-  if(it == kCorrectorSteps) publish_next_block(a, blockIdx.x, k, t);
+  return warp_sum(make_double2(f[0].x + f[1].x, f[0].y + f[1].y));
+}
+
+__device__ __forceinline__ void cluster_arrive_wait()
+{
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// v at the same shared-memory address in the cluster's block `rank`
+__device__ __forceinline__ void st_cluster(const double2 *p, int rank, double2 v)
+{
+  const unsigned own = (unsigned)__cvta_generic_to_shared(p);
+  unsigned there;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(own), "r"(rank));
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(there), "d"(v.x), "d"(v.y) : "memory");
+}
+
+// rows: dots per block; cache: near entries a block can hold (0: read the
+// list); stage: the grid form's iterates are copied into shared memory;
+// state_smem: so are the rows' states.
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kGroupThreads) step_group_kernel(StepArgs a, int k0, int k1, int rows, int cache,
+                                                                    int stage, int state_smem, double2 *gcur,
+                                                                    unsigned *counter)
+{
+  extern __shared__ double2 smem_group[];
+  double2 *cur = smem_group;                               // [2][n_pad] (cluster), [n_pad] (grid, staged)
+  double2 *ncoef = cur + (CLUSTER ? 2 : stage) * a.n_pad;  // [cache]
+  int *nidx = reinterpret_cast<int *>(ncoef + cache);      // [cache]
+  __shared__ int s_abort;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nb = gridDim.x;
+  const int row0 = blockIdx.x * rows, nrow = max(0, min(rows, a.n_pad - row0));
+  // [rows], after the cache (an even number of ints), or in global memory
+  RowState *state = state_smem ? reinterpret_cast<RowState *>(nidx + ((cache + 3) & ~3))
+                               : reinterpret_cast<RowState *>(gcur + 2 * (long long)a.n_pad) + row0;
+  const int t0 = *a.far_t0, nt = a.w.n_time;
+  const int E0 = nrow > 0 ? a.near_ptr[row0] : 0, E1 = nrow > 0 ? a.near_ptr[row0 + nrow] : 0;
+  if(cache > 0)
+    for(int e = E0 + threadIdx.x; e < E1; e += kGroupThreads) {
+      ncoef[e - E0] = a.near_coef[e];
+      nidx[e - E0] = a.near_idx[e];
+    }
+  if(threadIdx.x == 0) s_abort = 0;
+  for(int r = threadIdx.x; r < nrow; r += kGroupThreads) {
+    const int idx = row0 + r;
+    state[r].live = a.user[idx] >= 0;
+    state[r].dc = dot_const(a, idx, a.user[idx] >= 0);
+    state[r].e0 = a.near_ptr[idx] - (cache > 0 ? E0 : 0);
+    state[r].e1 = a.near_ptr[idx + 1] - (cache > 0 ? E0 : 0);
+  }
+  unsigned epoch = 0;
+  if(CLUSTER)
+    cluster_arrive_wait();  // every block has started before its memory is written
+  else
+    __syncthreads();
+  for(int k = k0; k < k1; ++k) {
+    const int t = t0 + k;
+    if(t >= a.T) break;  // uniform across the grid
+    // a warp per row: the sums over earlier steps
+    for(int r = w; r < nrow; r += kGroupWarps) {
+      RowState &st = state[r];
+      if(!st.live) continue;
+      const int idx = row0 + r;
+      const double2 m = group_past(a, idx, t);
+      // window sums, a lane per step of the window
+      double2 acc[4];
+#pragma unroll
+      for(int v = 0; v < 4; ++v) acc[v] = make_double2(0.0, 0.0);
+      if(lane < nt) {
+        const double2 *b = a.pcr + (long long)pc_slot(t - nt + lane) * 4 * a.n_pad + idx;
+        pc_term(a, a.w.ps, a.w.cs, nt, lane, b[0], b[a.n_pad], b[2 * a.n_pad], b[3 * a.n_pad], acc);
+      }
+#pragma unroll
+      for(int v = 0; v < 4; ++v) acc[v] = warp_sum(acc[v]);
+      if(lane == 0) {
+        const double2 F = a.far_field[(long long)k * a.n_pad + idx];
+        st.r[0] = acc[0];
+        st.r[1] = acc[1];
+        st.H[0] = acc[2];
+        st.H[1] = acc[3];
+        st.past = make_double2(F.x + m.x, F.y + m.y);
+      }
+    }
+    for(int r = threadIdx.x; r < nrow; r += kGroupThreads)
+      if(state[r].live) state[r].pul = pulse_rabi(a, row0 + r, t);
+    __syncthreads();
+    // evaluation `it` follows the exchange of iterate `it`
+    for(int it = 0;; ++it) {
+      // a thread per row: the evaluation of the last iterate and its correction
+      for(int r = threadIdx.x; r < nrow; r += kGroupThreads) {
+        RowState &st = state[r];
+        const int idx = row0 + r;
+        double2 v = make_double2(0.0, 0.0);
+        if(st.live) {
+          double2 x[2] = {st.r[0], st.r[1]};
+          if(it > 0) {
+            const double2 om =
+                make_double2((0.0 + st.pul) + (st.past.x + st.near.x), 0.0 + (st.past.y + st.near.y));
+            double2 dr[2];
+            liouville(x[0], x[1], om, st.dc, dr[0], dr[1]);
+            if(it > kCorrectorSteps) {
+              finish_state(a, idx, t, x, dr);
+              continue;
+            }
+            const double2 H[2] = {st.H[0], st.H[1]};
+            corrector(a, dr, H, x);
+            st.r[0] = x[0];
+            st.r[1] = x[1];
+          }
+          // the step's final iterate: the ring's value, read by the next step
+          if(it == kCorrectorSteps) finish_ring(a, idx, t, x);
+          v = prefactor(x[1], a.frame);
+        }
+        if(it > kCorrectorSteps) continue;
+        if(CLUSTER) {
+          for(int b = 0; b < nb; ++b) st_cluster(cur + (epoch & 1) * a.n_pad + idx, b, v);
+        } else {
+          __stcg(gcur + (long long)(epoch & 1) * a.n_pad + idx, v);
+        }
+      }
+      if(it > kCorrectorSteps) break;
+      const double2 *now;
+      if(CLUSTER) {
+        cluster_arrive_wait();
+        now = cur + (epoch & 1) * a.n_pad;
+      } else {
+        __syncthreads();
+        if(threadIdx.x == 0) {
+          post_step(counter);
+          const int limit = a.spin_limit > 0 ? a.spin_limit : kGridSpins;
+          int spins = 0;
+          while(ld_acquire(counter) < (epoch + 1) * nb) {
+            if(++spins > limit) {
+              s_abort = 1;
+              atomicMin(a.d_bad, -2);
+              break;
+            }
+          }
+        }
+        __syncthreads();
+        if(s_abort) return;  // uniform across the block; the others run out too
+        now = gcur + (long long)(epoch & 1) * a.n_pad;
+        if(stage) {
+          for(int i = threadIdx.x; i < a.n_pad; i += kGroupThreads) cur[i] = __ldcg(now + i);
+          __syncthreads();
+          now = cur;
+        }
+      }
+      // a warp per row: the sum over its coupled dots
+      for(int r = w; r < nrow; r += kGroupWarps) {
+        RowState &st = state[r];
+        if(!st.live) continue;
+        // kNearFlight entries per lane in flight
+        double2 part[kNearFlight];
+#pragma unroll
+        for(int u = 0; u < kNearFlight; ++u) part[u] = make_double2(0.0, 0.0);
+        const int *ni = cache > 0 ? nidx : a.near_idx;
+        const double2 *nc = cache > 0 ? ncoef : a.near_coef;
+        for(int e = st.e0 + lane; e < st.e1; e += 32 * kNearFlight) {
+          int b[kNearFlight];
+          double2 c[kNearFlight];
+#pragma unroll
+          for(int u = 0; u < kNearFlight; ++u) {
+            const int j = min(e + 32 * u, st.e1 - 1);
+            b[u] = ni[j];
+            c[u] = nc[j];
+          }
+#pragma unroll
+          for(int u = 0; u < kNearFlight; ++u) {
+            const double2 x = cmul(CLUSTER || stage ? now[b[u]] : __ldcg(now + b[u]), c[u]);
+            if(e + 32 * u < st.e1) {
+              part[u].x += x.x;
+              part[u].y += x.y;
+            }
+          }
+        }
+        static_assert(kNearFlight == 4, "sum of four");
+        const double2 nf = warp_sum(make_double2((part[0].x + part[1].x) + (part[2].x + part[3].x),
+                                                 (part[0].y + part[1].y) + (part[2].y + part[3].y)));
+        if(lane == 0) st.near = nf;
+      }
+      __syncthreads();
+      ++epoch;
+    }
+    if(k == kTimeBlock - 1 && blockIdx.x == 0 && threadIdx.x == 0) *a.d_next = t + 1;
+    __syncthreads();
+  }
+  if(CLUSTER) cluster_arrive_wait();  // no block leaves while another may write to it
+}
+
+static size_t group_smem(const GroupShape &g, int n_pad)
+{
+  return sizeof(double2) * ((size_t)(g.cluster ? 2 : g.stage) * n_pad + g.cache) +
+         sizeof(int) * (size_t)((g.cache + 3) & ~3) + (g.state ? sizeof(RowState) * (size_t)g.rows : 0);
+}
+
+// Shared memory a block of the general form may take: the device's limit less
+// the kernel's static part.  The attribute is the same for every handle.
+static size_t group_room()
+{
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  const size_t room = (size_t)optin - 1024;
+  cudaFuncSetAttribute(step_group_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
+  cudaFuncSetAttribute(step_group_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaFuncSetAttribute(step_group_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
+  return room;
+}
+
+// The launch's shape for an ensemble (near_ptr: its near list, CSR by dot).
+// One cluster of up to 16 blocks while that gives every dot a warp of its own
+// (two dots a warp took 115 us a step at 400 dots, the grid of one each 78 at
+// 512).  Else a grid of one block per SM, its rows' states, the iterates and
+// the near lists in shared memory as far as they fit.
+GroupShape group_shape(int n_pad, const int *near_ptr)
+{
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const size_t room = group_room();
+  auto shape = [&](int blocks) {
+    GroupShape g{};
+    g.blocks = blocks;
+    g.rows = (n_pad + blocks - 1) / blocks;
+    for(int b = 0; b < blocks; ++b) {
+      const int lo = b * g.rows < n_pad ? b * g.rows : n_pad, hi = lo + g.rows < n_pad ? lo + g.rows : n_pad;
+      const int e = near_ptr[hi] - near_ptr[lo];
+      if(e > g.cache) g.cache = e;
+    }
+    return g;
+  };
+  const int blocks = n_pad >= 8 * kClusterBlocks ? kClusterBlocks : kClusterBlocks / 2;
+  if(blocks * kGroupWarps >= n_pad) {
+    GroupShape g = shape(blocks);
+    g.cluster = 1;
+    g.state = 1;
+    g.smem = group_smem(g, n_pad);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kGroupThreads);
+    cfg.dynamicSmemBytes = g.smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = blocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if(g.smem <= room && cudaOccupancyMaxActiveClusters(&fit, step_group_kernel<true>, &cfg) == cudaSuccess && fit > 0)
+      return g;
+    cudaGetLastError();
+  }
+  const int want = (n_pad + kGroupWarps - 1) / kGroupWarps;
+  GroupShape g = shape(want < sms ? want : sms);
+  const int cache = g.cache;
+  g.cache = 0;
+  g.state = 1;
+  if(group_smem(g, n_pad) > room) g.state = 0;
+  g.stage = 1;
+  if(group_smem(g, n_pad) > room) g.stage = 0;
+  g.cache = cache;
+  if(group_smem(g, n_pad) > room) g.cache = 0;
+  g.smem = group_smem(g, n_pad);
+  return g;
+}
+
+void launch_step_group(const StepArgs &a, int k0, int k1, const GroupShape &g, unsigned *counter, void *stream)
+{
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g.blocks);
+  cfg.blockDim = dim3(kGroupThreads);
+  cfg.dynamicSmemBytes = g.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if(g.cluster) {
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = g.blocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchKernelEx(&cfg, step_group_kernel<true>, a, k0, k1, g.rows, g.cache, g.stage, g.state, a.scratch,
+                       counter);
+  } else {
+    cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cudaLaunchKernelEx(&cfg, step_group_kernel<false>, a, k0, k1, g.rows, g.cache, g.stage, g.state, a.scratch,
+                       counter);
+  }
 }
 
 void launch_step_fused(const StepArgs &a, int k, int nblocks, void *stream)
@@ -1133,12 +1423,6 @@ void launch_step_fused(const StepArgs &a, int k, int nblocks, void *stream)
     step_fused_kernel<22><<<nblocks, 32 * kParts, 0, s>>>(a, k);
   else
     step_fused_kernel<0><<<nblocks, 32 * kParts, 0, s>>>(a, k);
-}
-
-void launch_step_general(const StepArgs &a, int k, int phase, void *stream)
-{
-  const int nblocks = (a.n_pad + kStepBlock - 1) / kStepBlock;
-  step_general_kernel<<<nblocks, kStepBlock, 0, (cudaStream_t)stream>>>(a, k, phase);
 }
 
 // HistoryInteraction::evaluate at an explicit step: past partial sums plus
