@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -91,6 +92,7 @@ struct qg_handle_s {
   int traj_k = 0;
   double2 *d_io = nullptr;    // N complex device staging for evaluate / set_history
   double2 *h_io = nullptr;    // pinned N complex, made at the first evaluate / history copy
+  char *box = nullptr;        // pinned box of small results: the bad step, then rows or fields
 
   bool fused = true;
   int step_blocks = 0;
@@ -108,6 +110,7 @@ struct qg_handle_s {
   int far_block = -0x7fffffff;  // first step of the far block the partials hold
   double table_ms = 0;
   int next_step = 0;
+  int dev_next = -1;  // what d_ints[0] holds, as far as the host knows (-1: unknown)
   int eval_cached = -0x7fffffff;
 
   // K-step block graphs by the far kernel's form, [traj off, traj on] each
@@ -322,6 +325,42 @@ static void pool_free(qg_handle *h, void *p)
     cudaFree(p);
 }
 
+// ---- pinned boxes ---------------------------------------------------------------
+// Small results (a few recorded steps, an evaluation, the first bad step) go
+// through a pinned box of the handle, which kernels and copies reach without
+// the driver's staging of pageable memory.  A pinned allocation costs about a
+// millisecond, so boxes of destroyed handles are kept for the next ones, at
+// most kBoxesKept of them for the process.
+constexpr size_t kBoxBytes = 256 << 10;
+constexpr size_t kBoxesKept = 16;
+static std::mutex g_box_mu;
+static std::vector<void *> g_boxes;
+
+static cudaError_t take_box(void **p)
+{
+  {
+    std::lock_guard<std::mutex> lock(g_box_mu);
+    if(!g_boxes.empty()) {
+      *p = g_boxes.back();
+      g_boxes.pop_back();
+      return cudaSuccess;
+    }
+  }
+  return cudaHostAlloc(p, kBoxBytes, cudaHostAllocPortable | cudaHostAllocMapped);
+}
+
+static void give_box(void *p)
+{
+  {
+    std::lock_guard<std::mutex> lock(g_box_mu);
+    if(g_boxes.size() < kBoxesKept) {
+      g_boxes.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
 template <typename T>
 static qg_status dalloc(qg_handle *h, T **p, size_t count)
 {
@@ -372,6 +411,7 @@ static void destroy_handle(qg_handle *h)
   }
   for(void *p : h->allocs) pool_free(h, p);
   if(h->h_io) cudaFreeHost(h->h_io);
+  if(h->box) give_box(h->box);
   if(h->stream) cudaStreamDestroy(h->stream);
   if(h->copy_stream) cudaStreamDestroy(h->copy_stream);
   delete h;
@@ -769,6 +809,7 @@ static qg_status reset_state(qg_handle *h)
   h->eval_cached = -0x7fffffff;
   h->far_block = -0x7fffffff;
   h->ring_clean = true;
+  h->dev_next = 0;
   return QG_OK;
 }
 
@@ -1279,20 +1320,23 @@ static void enqueue_far(qg_handle *h, int t0, bool at_boundary, cudaEvent_t ea, 
 }
 
 // Steps k0 .. k1-1 of the current block in one launch.
-static void enqueue_step_block(qg_handle *h, int k0, int k1, bool traj)
+// traj_t0: the recorded rows' first step (INT_MIN: read from d_ints[3]).
+static void enqueue_step_block(qg_handle *h, int k0, int k1, bool traj, int traj_t0 = INT_MIN)
 {
   StepArgs a = h->step_args(!h->fused);
   if(traj) a.traj = h->d_traj;
+  if(traj_t0 != INT_MIN) a.traj_t0 = nullptr, a.traj_base = traj_t0;
   if(h->fused)
     launch_step_block(a, k0, k1, h->step_blocks, h->d_flags, h->stream);
   else
     launch_step_group(a, k0, k1, h->group_launch, h->d_flags, h->stream);
 }
 
-static void enqueue_dot_step(qg_handle *h, int k, bool traj)
+static void enqueue_dot_step(qg_handle *h, int k, bool traj, int traj_t0 = INT_MIN)
 {
   StepArgs a = h->step_args(!h->fused);
   if(traj) a.traj = h->d_traj;
+  if(traj_t0 != INT_MIN) a.traj_t0 = nullptr, a.traj_base = traj_t0;
   if(h->fused)
     launch_step_fused(a, k, h->shard_world > 1 ? h->blk_hi - h->blk_lo : h->step_blocks, h->stream);
   else
@@ -1397,11 +1441,22 @@ static qg_status collect_events(qg_handle *h, int nev, int nstep)
   return QG_OK;
 }
 
-// Enqueues steps [t, t + count); whole aligned blocks replay the graph.
-static qg_status launch_steps(qg_handle *h, int t, int count, bool traj)
+// Enqueues steps [t, t + count); whole aligned blocks replay the graph.  traj:
+// record the steps, step traj_t0 into row 0.
+static qg_status launch_steps(qg_handle *h, int t, int count, bool traj, int traj_t0 = 0)
 {
+  if(count <= 0) return QG_OK;
   int nev = 0, nstep = 0;
-  if(count > 0 && t % kTimeBlock == 0) launch_set_int(h->d_ints + 0, t, h->stream);
+  // the far launch at a boundary reads its first step from d_ints[0], which
+  // the previous block's last step kernel has set
+  if(t % kTimeBlock == 0 && h->dev_next != t) {
+    launch_set_int(h->d_ints + 0, t, h->stream);
+    h->dev_next = t;
+  }
+  if((t + count) / kTimeBlock > t / kTimeBlock) h->dev_next = (t + count) / kTimeBlock * kTimeBlock;
+  // a block graph reads the rows' first step from the device, a launch of its
+  // own gets it as an argument
+  if(traj && h->use_graph && (t % kTimeBlock + count) >= kTimeBlock) launch_set_int(h->d_ints + 3, traj_t0, h->stream);
   while(count > 0) {
     const int t0 = t - t % kTimeBlock;
     if(t == t0 && count >= kTimeBlock && h->use_graph) {
@@ -1427,9 +1482,9 @@ static qg_status launch_steps(qg_handle *h, int t, int count, bool traj)
     const int span = h->block_step || !h->fused ? std::min(count, t0 + kTimeBlock - t) : 1;
     if(h->profile) cudaEventRecord(h->ev_c[nstep], h->stream);
     if(span > 1)
-      enqueue_step_block(h, t - t0, t - t0 + span, traj);
+      enqueue_step_block(h, t - t0, t - t0 + span, traj, traj_t0);
     else
-      enqueue_dot_step(h, t - t0, traj);
+      enqueue_dot_step(h, t - t0, traj, traj_t0);
     if(h->profile) cudaEventRecord(h->ev_d[nstep++], h->stream);
     if(h->profile && (nev == 256 || nstep == 256)) {
       QG_TRY(collect_events(h, nev, nstep));
@@ -1553,6 +1608,12 @@ extern "C" qg_status qg_shard_import(qg_handle *h, const double *d_full)
   return QG_OK;
 }
 
+static qg_status ensure_box(qg_handle *h)
+{
+  if(!h->box) QG_CUDA(take_box((void **)&h->box));
+  return QG_OK;
+}
+
 extern "C" qg_status qg_run(qg_handle *h, int n_steps, double *rho_out, int *bad_step)
 {
   if(!h) return qg_fail(QG_ERR_INVALID_ARG, "qg_run: NULL handle");
@@ -1572,8 +1633,18 @@ extern "C" qg_status qg_run(qg_handle *h, int n_steps, double *rho_out, int *bad
   const int t_start = h->next_step;
   h->eval_cached = -0x7fffffff;
   const size_t row = (size_t)h->n * 2;  // double2 per step
+  const bool small = rho_out && n_steps <= h->traj_k && sizeof(double2) * row * (size_t)n_steps <= kBoxBytes - 64;
+  if(small) QG_TRY(ensure_box(h));
+  int bad = kBadNone;
+  int *bad_at = h->box ? reinterpret_cast<int *>(h->box) : &bad;
+  char *box_rows = h->box + 64;
   if(!rho_out) {
     QG_TRY(launch_steps(h, t_start, n_steps, false));
+  } else if(small) {
+    // a few rows: one copy into the pinned box on the same stream
+    QG_TRY(launch_steps(h, t_start, n_steps, true, t_start));
+    QG_CUDA(cudaMemcpyAsync(box_rows, h->d_traj, sizeof(double2) * row * (size_t)n_steps, cudaMemcpyDeviceToHost,
+                            h->stream));
   } else {
     // Every step's state straight into the caller's buffer.  Chunks of
     // traj_k steps alternate between the two halves of d_traj.  Chunk c's
@@ -1600,8 +1671,7 @@ extern "C" qg_status qg_run(qg_handle *h, int n_steps, double *rho_out, int *bad
       const int k = std::min(K, n_steps - c * K);
       if(c >= 2) ce = cudaStreamWaitEvent(h->stream, h->ev_copy[b], 0);
       if(ce != cudaSuccess) break;
-      launch_set_int(h->d_ints + 3, t_start + c * K - b * K, h->stream);
-      st = launch_steps(h, t_start + c * K, k, true);
+      st = launch_steps(h, t_start + c * K, k, true, t_start + c * K - b * K);
       if(st != QG_OK) break;
       ce = cudaEventRecord(h->ev_chunk[b], h->stream);
       if(ce == cudaSuccess && c >= 1) ce = copy_out(c - 1);
@@ -1613,10 +1683,11 @@ extern "C" qg_status qg_run(qg_handle *h, int n_steps, double *rho_out, int *bad
     QG_CUDA(ce);
     QG_CUDA(ce2);
   }
-  int bad = kBadNone;
-  QG_CUDA(cudaMemcpyAsync(&bad, h->d_ints + 2, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  QG_CUDA(cudaMemcpyAsync(bad_at, h->d_ints + 2, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   QG_CUDA(cudaStreamSynchronize(h->stream));
   QG_CUDA(cudaGetLastError());
+  bad = *bad_at;
+  if(small) std::memcpy(rho_out, box_rows, sizeof(double2) * row * (size_t)n_steps);
   h->next_step = t_start + n_steps;
   if(bad == -2)
     return qg_fail(QG_ERR_CUDA, "qg_run: a wait in the step kernel timed out");
@@ -1741,6 +1812,7 @@ extern "C" qg_status qg_batch_add(qg_batch *b, qg_handle *h)
   b->frame = h->params.frame;
   b->n_time = h->w.n_time;
   // the member's device state must name the next block's first step
+  h->dev_next = -1;
   QG_CUDA(cudaStreamSynchronize(h->stream));
   launch_set_int(h->d_ints + 0, h->next_step, b->stream);
   b->members.push_back(h);
@@ -1948,6 +2020,7 @@ extern "C" qg_status qg_batch_run(qg_batch *b, int n_blocks)
     h->eval_cached = -0x7fffffff;
     h->batch_bad = b->h_bad_all[e];
     h->batch_bad_valid = true;
+    h->dev_next = -1;
   }
   return QG_OK;
 }
@@ -2186,6 +2259,7 @@ extern "C" qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t by
   h->far_block = -0x7fffffff;
   h->eval_cached = -0x7fffffff;
   h->ring_clean = clean;
+  h->dev_next = -1;
   return QG_OK;
 }
 
@@ -2229,10 +2303,26 @@ extern "C" qg_status qg_history_evaluate(qg_handle *h, int step, const double *r
     return qg_fail(QG_ERR_INVALID_ARG, "qg_history_evaluate: step %d outside [0, %d)", step, h->T);
   QG_CUDA(cudaSetDevice(h->device));
   StepArgs a = h->step_args(true);
+  // small ensembles: the kernels read the iterate from, and write the field
+  // to, the handle's pinned box (dot by dot over the bus: copies are cheaper
+  // from some thousand dots on)
+  const size_t bytes = sizeof(double2) * (size_t)h->n;
+  const bool small = h->n <= 1024;
+  static_assert(2 * sizeof(double2) * 1024 <= kBoxBytes, "box");
+  if(small) QG_TRY(ensure_box(h));
+  const double2 *in = h->d_io;
+  double2 *out = h->d_io;
+  if(small) {
+    in = reinterpret_cast<const double2 *>(h->box);
+    out = reinterpret_cast<double2 *>(h->box + kBoxBytes / 2);
+  }
   if(rho01_step) {
-    QG_TRY(upload_io(h, rho01_step));
+    if(small)
+      std::memcpy(h->box, rho01_step, bytes);
+    else
+      QG_TRY(upload_io(h, rho01_step));
     h->ring_clean = false;
-    launch_ring_write(a, step, h->d_io, h->stream);
+    launch_ring_write(a, step, in, h->stream);
     launch_ring32_rebuild(a, h->stream);
   }
   if(h->eval_cached != step) {
@@ -2243,9 +2333,12 @@ extern "C" qg_status qg_history_evaluate(qg_handle *h, int step, const double *r
     h->far_block = -0x7fffffff;
   }
   a.far_t0 = h->d_ints + 4;
-  launch_eval_field(a, h->d_ints + 4, h->d_io, h->stream);
+  launch_eval_field(a, h->d_ints + 4, out, h->stream);
   QG_CUDA(cudaGetLastError());
-  return download_io(h, field_out);
+  if(!small) return download_io(h, field_out);
+  QG_CUDA(cudaStreamSynchronize(h->stream));
+  std::memcpy(field_out, out, bytes);
+  return QG_OK;
 }
 
 extern "C" qg_status qg_history_evaluate_noalloc(qg_handle *h, int step, const double *d_rho01_step,

@@ -188,7 +188,8 @@ struct StepArgs {
     double2 *scratch;      // general form: [2][n_pad] iterates exchanged by its grid, then kRowStateBytes a dot
   double2 *traj;         // [k][n][2] user order or null
   int traj_rows;         // rows allocated in traj
-  const int *traj_t0;
+  const int *traj_t0;    // the step of row 0 (null: traj_base)
+  int traj_base;
   int *d_next;           // first step of the next far block (set by the last
                          // step kernel of a block, read by the far kernel)
   int *d_bad;

@@ -182,7 +182,7 @@ __device__ __forceinline__ void finish_state(const StepArgs &a, int idx, int t, 
   base[2 * a.n_pad] = dr[0];
   base[3 * a.n_pad] = dr[1];
   if(a.traj) {
-    const int row = t - *a.traj_t0;
+    const int row = t - (a.traj_t0 ? *a.traj_t0 : a.traj_base);
     if(row >= 0 && row < a.traj_rows) {
       double2 *tr = a.traj + ((long long)row * a.n + a.user[idx]) * 2;
       tr[0] = r[0];
