@@ -792,6 +792,15 @@ static qg_status build_lists(qg_handle *h, const TableArgs &ta)
   return QG_OK;
 }
 
+// The step kernels' flags start alike (a launch that gave up a wait leaves them
+// apart).
+static qg_status clear_flags(qg_handle *h)
+{
+  QG_CUDA(cudaMemsetAsync(h->d_flags, 0, sizeof(unsigned) * (size_t)std::max(h->step_blocks, 1) * kFlagStride,
+                          h->stream));
+  return QG_OK;
+}
+
 static qg_status reset_state(qg_handle *h)
 {
   h->batch_bad_valid = false;
@@ -802,6 +811,7 @@ static qg_status reset_state(qg_handle *h)
   }
   QG_CUDA(cudaMemsetAsync(h->d_field, 0, sizeof(double2) * (size_t)kTimeBlock * h->n_pad, h->stream));
   launch_init_state(h->step_args(false), h->stream);
+  QG_TRY(clear_flags(h));
   int init[9] = {0, 0, kBadNone, 0, 0, h->max_delay, 0, 0, 0};
   QG_CUDA(cudaMemcpyAsync(h->d_ints, init, sizeof init, cudaMemcpyHostToDevice, h->stream));
   QG_CUDA(cudaStreamSynchronize(h->stream));
@@ -2254,6 +2264,7 @@ extern "C" qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t by
   }
   QG_CUDA(cudaMemcpyAsync(h->d_pcr, p, hd.pcr_bytes, cudaMemcpyHostToDevice, h->stream));
   QG_CUDA(cudaMemcpyAsync(h->d_ints + 2, &hd.bad, sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  QG_TRY(clear_flags(h));
   QG_CUDA(cudaStreamSynchronize(h->stream));
   h->next_step = hd.next_step;
   h->far_block = -0x7fffffff;

@@ -600,7 +600,8 @@ void launch_step_batch(const StepArgs *args, const int *block_off, int n_ens, in
 // partners' history of step k-1 and earlier, so the helpers first wait until
 // every block that holds one of the block's mid-list partners (and the block
 // itself) has finished step k-1.  Each block counts its finished steps in
-// flags[block * kFlagStride] (zeroed before the launch); warp 0 posts a step
+// flags[block * kFlagStride] (which count on from launch to launch: a launch
+// that ends posts the same steps on every block); warp 0 posts a step
 // as soon as its rho01 is stored.  The post is on the critical path between
 // blocks (a partner's post, then the helpers' work, bounds the step), so
 // warp 0 posts it itself: handing it to another warp through a barrier
@@ -655,7 +656,7 @@ __device__ __forceinline__ bool wait_blocks(const unsigned *flags, const int *li
   for(int i = threadIdx.x & 31; i < n && ok; i += 32) {
     const unsigned *f = flags + (long long)__ldg(list + i) * kFlagStride;
     int spins = 0;
-    while(ld_acquire(f) < target) {
+    while((int)(ld_acquire(f) - target) < 0) {
       if(++spins > max_spins) {
         ok = false;
         break;
@@ -836,31 +837,47 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 2) step_block_kernel(StepArg
   const int B0 = a.pb_ptr[blk], NB = a.pb_ptr[blk + 1] - B0;  // blocks holding this block's partners
 
   // prologue: window, weights, the launch's far field and pulse, prev01, and
-  // the block's mid list and partner history when they fit.  The copies are
-  // latency-bound (one L2 round trip each), so each thread issues several
-  // independent loads before it stores any.
-  constexpr int kPro = 4;  // loads in flight per thread in the copy loops
-  for(int sl = part; sl < kPcDepth; sl += kBlockWarps) {
-    double2 v[4];
-#pragma unroll
-    for(int c = 0; c < 4; ++c) v[c] = a.pcr[((long long)sl * 4 + c) * a.n_pad + idx];
-#pragma unroll
-    for(int c = 0; c < 4; ++c) m.win[sl][c][lane] = v[c];
-  }
-  for(int i = threadIdx.x; i < 2 * nt; i += blockDim.x) {
-    m.ps[i] = a.w.ps[i];
-    m.cs[i] = a.w.cs[i];
-  }
+  // the block's mid list and partner history when they fit.  It is bound by
+  // the latency of its reads (an L2 round trip each), so every thread issues
+  // its reads of the window, the far field and the dot together before it
+  // stores any, and several at a time in the lists' loops.
+  constexpr int kPro = 4;  // loads in flight per thread in the lists' loops
+  constexpr int kWinLoads = (kPcDepth + kBlockWarps - 1) / kBlockWarps, kFarLoads = kTimeBlock / kBlockWarps;
+  // the flags count on from launch to launch; every block's stands alike here
+  const unsigned posted = ld_acquire(flags + (long long)blk * kFlagStride);
   {
+    double2 v[kWinLoads][4], far[kFarLoads];
+#pragma unroll
+    for(int u = 0; u < kWinLoads; ++u)
+#pragma unroll
+      for(int c = 0; c < 4; ++c)
+        v[u][c] = a.pcr[((long long)min(part + u * kBlockWarps, kPcDepth - 1) * 4 + c) * a.n_pad + idx];
+#pragma unroll
+    for(int u = 0; u < kFarLoads; ++u)
+      far[u] = a.far_field[(long long)min(k0 + part + u * kBlockWarps, kTimeBlock - 1) * a.n_pad + idx];
+    const double2 prev = a.ring[(long long)idx * a.stride + ring_slot(t0 + k0 - 1, a.W)];
     // the pulse from the dot's k.r and dipole, loaded once (pulse_rabi's
     // operations)
     const double kr = live ? pulse_kr(a, idx) : 0.0;
     const double d0 = live ? a.dip[3 * idx] : 0.0, d1 = live ? a.dip[3 * idx + 1] : 0.0,
                  d2 = live ? a.dip[3 * idx + 2] : 0.0;
-    for(int kk = k0 + part; kk < k1; kk += kBlockWarps) {
-      m.far[kk * BS + lane] = live ? a.far_field[(long long)kk * a.n_pad + idx] : make_double2(0.0, 0.0);
-      m.pul[kk * BS + lane] = live ? pulse_at(a, kr, d0, d1, d2, t0 + kk) : 0.0;
+    for(int i = threadIdx.x; i < 2 * nt; i += blockDim.x) {
+      m.ps[i] = a.w.ps[i];
+      m.cs[i] = a.w.cs[i];
     }
+#pragma unroll
+    for(int u = 0; u < kFarLoads; ++u) {
+      const int kk = k0 + part + u * kBlockWarps;
+      if(kk >= k1) continue;
+      m.pul[kk * BS + lane] = live ? pulse_at(a, kr, d0, d1, d2, t0 + kk) : 0.0;
+      m.far[kk * BS + lane] = live ? far[u] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for(int u = 0; u < kWinLoads; ++u)
+#pragma unroll
+      for(int c = 0; c < 4; ++c)
+        if(part + u * kBlockWarps < kPcDepth) m.win[part + u * kBlockWarps][c][lane] = v[u][c];
+    if(part == 0) m.prev01[lane] = prev;
   }
   const int E0 = a.mid_ptr[blk * BS], E = a.mid_ptr[blk * BS + BS] - E0;
   const bool cached = E <= a.mid_cache;
@@ -914,7 +931,6 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 2) step_block_kernel(StepArg
       }
     }
   }
-  if(part == 0) m.prev01[lane] = a.ring[(long long)idx * a.stride + ring_slot(t0 + k0 - 1, a.W)];
   if(threadIdx.x == 0) s_abort = 0;
   BlockConst bc;
   bc.live = live;
@@ -937,7 +953,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 2) step_block_kernel(StepArg
     const int buf = k & 1;
     if(part == 0) {
       bool ok = true;
-      if(!a.lag && k > k0) ok = wait_blocks(flags, a.pb_idx + B0, NB, k - k0, a.spin_limit);  // partners' step t-1
+      if(!a.lag && k > k0) ok = wait_blocks(flags, a.pb_idx + B0, NB, posted + (k - k0), a.spin_limit);  // partners' step t-1
       if(ok) {
         double2 P[2], H[2], r[2], dr[2], past = make_double2(0.0, 0.0);
         double pul = 0;
@@ -985,7 +1001,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 2) step_block_kernel(StepArg
       }
     } else if(helper && k + 1 < k1 && t + 1 < a.T) {
       // step k+1's sums; M_old needs the partner blocks' step k-1
-      if(hw == 0 && k > k0 && !wait_blocks(flags, a.pb_idx + B0, NB, k - k0, a.spin_limit) && lane == 0) {
+      if(hw == 0 && k > k0 && !wait_blocks(flags, a.pb_idx + B0, NB, posted + (k - k0), a.spin_limit) && lane == 0) {
         s_abort = 1;
         atomicMin(a.d_bad, -2);
       }
@@ -1007,7 +1023,6 @@ void launch_step_block(const StepArgs &a, int k0, int k1, int nblocks, unsigned 
   cudaStream_t s = (cudaStream_t)stream;
   const size_t smem = block_smem_bytes(a.q, a.mid_cache, a.hist_cap);
   step_block_attrs(smem);
-  cudaMemsetAsync(flags, 0, sizeof(unsigned) * nblocks * kFlagStride, s);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nblocks);
   cfg.blockDim = dim3(32 * kBlockWarps);
