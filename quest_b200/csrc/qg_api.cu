@@ -951,7 +951,15 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
       return qg_fail(QG_ERR_UNSUPPORTED, "qg_create: weights.n_time %d exceeds the 22-step window",
                      wt.n_time);
   } else {
-    QG_TRY(qg_pc_weights(18, 22, 3.15, &wt));
+    // the default weights are the same for every handle and take milliseconds
+    // to solve for: once per process
+    static const std::pair<qg_status, qg_weights> standard = [] {
+      qg_weights w;
+      const qg_status st = qg_pc_weights(18, 22, 3.15, &w);
+      return std::make_pair(st, w);
+    }();
+    QG_TRY(standard.first);
+    wt = standard.second;
   }
   h->w.n_time = wt.n_time;
   for(int i = 0; i < 2 * wt.n_time; ++i) {
