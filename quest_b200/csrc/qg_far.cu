@@ -25,8 +25,8 @@
 // their windows, at the 32 different delays d(a_l, b), fall in one short
 // stretch of b's history row: a handful of cache lines per load instead of
 // 32.  The table's entries are copied asynchronously into the warp's own
-// shared memory three sources ahead (FP64) or prefetched in registers
-// (mixed), the delays five sources ahead.  A warp none of whose windows
+// shared memory (FP64) or prefetched in registers (mixed), a source ahead, the
+// delays earlier still.  A warp none of whose windows
 // reaches step -22 yet skips the source, its coefficients included, so the
 // first blocks of a run cost what they use.
 //
@@ -62,20 +62,32 @@ namespace qg {
 template <bool MIXED>
 constexpr int kFarBlocks = MIXED ? 4 : 3;
 
-// FP64: each lane copies its own entry of a source's q+1 coefficient rows into
-// its warp's stage (cp.async, evict-first in L2: the table is streamed once
-// per launch, the history ring should stay), P - 1 sources ahead.
-constexpr int kFarStages = 3;
+// FP64: each lane copies its own entries of the table into its warp's shared
+// memory: a source's q+1 coefficients one source ahead (evict-first in L2: the
+// table is streamed once per launch, the history ring should stay), its delay
+// kDelayAhead sources ahead.  Delays prefetched in registers are moved from
+// one to the next on every source, and the move waits for the load: a source
+// that every window skips cost 0.9 us.  First block of 4096 dots 284 -> 252 us,
+// a steady launch 642 -> 632 us, of 1500 dots 114 -> 111 us.  Coefficients two
+// sources ahead leave less to L1: 642 instead of 627 us at 4096 dots.
+constexpr int kDelayAhead = 4;
+constexpr int kDelaySlots = 8;
 
 template <int Q>
 struct FarStage {
-  double2 coef[kFarStages][Q + 1][32];
+  double2 coef[2][Q + 1][32];
+  int delay[kDelaySlots][32];
 };
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src, unsigned long long pol)
 {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "l"(pol) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *dst, const void *src, unsigned long long pol)
+{
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "l"(pol) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -87,12 +99,18 @@ __device__ __forceinline__ void cp_async_wait()
 template <int Q, bool LAB, bool MIXED, int FORM>
 struct FarBody;
 
+// Each lane reads back only what it copied.  One group of copies per source:
+// group s holds the coefficients of source s + 1 and the delays of source
+// s + kDelayAhead, so with all but the newest kDelayAhead - 2 groups done the
+// delays of source s + 1 are there, and with all but the newest one the
+// coefficients of source s.
 template <int Q, bool LAB, int FORM>
 struct FarBody<Q, LAB, false, FORM> {
   using Shared = FarStage<Q>;
   static __device__ __forceinline__ void run(const FarArgs &a, const FarTask &t, int t0, Shared &st)
   {
-    constexpr int K = kTimeBlock, P = kFarStages;
+    constexpr int K = kTimeBlock;
+    static_assert(kDelayAhead > 2 && kDelaySlots > kDelayAhead, "a slot is read before it is copied to again");
     using Acc = FarAcc<LAB, K>;
     const int lane = threadIdx.x & 31;
     // a window of delay d has a sample at step -22 or later
@@ -102,37 +120,47 @@ struct FarBody<Q, LAB, false, FORM> {
     const long long tile = (long long)t.I * a.nT;
     // a tile row's delays are one array over the sources, 32 entries each
     const int *dp = a.delay + tile * kTilePairs + lane;
-    auto load_delay = [&](int s) { return s < t.s1 ? __ldcs(dp + s * kTile) : -1; };
-    auto live = [&](int d) { return d >= K && d <= d_last; };
-    auto issue = [&](int s, int d) {
-      if(__any_sync(0xffffffffu, live(d))) {
-        const double2 *src = a.coef + ((tile + s / kTile) * (Q + 1)) * kTilePairs + (s % kTile) * kTile + lane;
-        double2(&dst)[Q + 1][32] = st.coef[s % P];
+    auto fetch_delay = [&](int s) {
+      if(s < t.s1) cp_async4(&st.delay[s % kDelaySlots][lane], dp + s * kTile, pol);
+    };
+    // the delay of source s, -1 where no window is to be read
+    auto delay = [&](int s) {
+      if(s >= t.s1) return -1;
+      const int d = st.delay[s % kDelaySlots][lane];
+      return d >= K && d <= d_last ? d : -1;
+    };
+    auto fetch_coef = [&](int s, int d) {
+      if(!__any_sync(0xffffffffu, d >= 0)) return;
+      const double2 *src = a.coef + ((tile + s / kTile) * (Q + 1)) * kTilePairs + (s % kTile) * kTile + lane;
 #pragma unroll
-        for(int i = 0; i <= Q; ++i) cp_async16(&dst[i][lane], src + i * kTilePairs, pol);
-      }
-      cp_async_commit();
+      for(int i = 0; i <= Q; ++i) cp_async16(&st.coef[s & 1][i][lane], src + i * kTilePairs, pol);
     };
     Acc acc;
     acc.zero();
-    int d0 = load_delay(t.s0), d1 = load_delay(t.s0 + 1), d2 = load_delay(t.s0 + 2), d3 = load_delay(t.s0 + 3),
-        d4 = load_delay(t.s0 + 4);
-    issue(t.s0, d0);
-    issue(t.s0 + 1, d1);
+#pragma unroll
+    for(int s = 0; s < kDelayAhead; ++s) fetch_delay(t.s0 + s);
+    cp_async_commit();
+    cp_async_wait<0>();
+    int d0 = delay(t.s0);
+    fetch_coef(t.s0, d0);
+    cp_async_commit();
 #pragma unroll 1
     for(int s = t.s0; s < t.s1; ++s) {
-      issue(s + 2, d2);
-      const int d5 = load_delay(s + 5);
-      cp_async_wait<P - 1>();  // each lane reads back only what it copied
-      if(live(d0)) {
+      cp_async_wait<kDelayAhead - 2>();
+      const int d1 = delay(s + 1);
+      fetch_coef(s + 1, d1);
+      fetch_delay(s + kDelayAhead);
+      cp_async_commit();
+      cp_async_wait<1>();
+      if(d0 >= 0) {
         typename Acc::C c[Q + 1];
 #pragma unroll
-        for(int i = 0; i <= Q; ++i) c[i] = Acc::from(st.coef[s % P][i][lane]);
+        for(int i = 0; i <= Q; ++i) c[i] = Acc::from(st.coef[s & 1][i][lane]);
         const int tau0 = t0 - d0 - Q;
         window_conv<Q, LAB, K, FORM>(a.ring + (long long)s * a.stride, wrap_slot(tau0, a.W), tau0, c, acc);
       }
       __syncwarp();
-      d0 = d1, d1 = d2, d2 = d3, d3 = d4, d4 = d5;
+      d0 = d1;
     }
     cp_async_wait<0>();
     store_partial<K>(a, t, acc);
@@ -257,8 +285,8 @@ void launch_far_reduce(const FarArgs &a, int steps, void *stream)
 }
 
 // ---- launches ----------------------------------------------------------------------
-// The stages' dynamic shared memory (37 KB a block at q = 5, 49 KB at q = 7,
-// above the default limit) is opted in once per function and device.
+// The stages' dynamic shared memory (28 KB a block at q = 5) is opted in once
+// per function and device.
 template <int Q, bool MIXED>
 constexpr size_t far_smem_bytes()
 {
