@@ -498,7 +498,11 @@ __device__ __forceinline__ void step_fused_body(const StepArgs &a, int blk, int 
   // launch_step_batch, nothing in others).
   cudaGridDependencySynchronize();
   const int t = *a.far_t0 + k;
-  if(t >= a.T) return;  // past this ensemble's last step (uniform per block)
+  if(t >= a.T) {  // past this ensemble's last step (uniform per block)
+    // an ensemble that ends within a block starts no block again
+    if(t - k < a.T) publish_next_block(a, blk, k, t);
+    return;
+  }
 
   // warp 0's inputs, requested before the gathers complete
   double2 F = make_double2(0.0, 0.0), Mn = F, T[4];

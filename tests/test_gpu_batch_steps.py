@@ -29,3 +29,20 @@ def test_overlapping_step_launches_keep_the_order(golden_weights, sizes, steps, 
     batch.close()
     for s in sims:
         s.close()
+
+
+def test_member_ending_within_a_block_keeps_its_state(golden_weights):
+    """Blocks run after such a member's last step change nothing of it."""
+    ens = [ensemble(80 + i, 200, 0.1, s, 5.0) for i, s in enumerate((64, 17, 24, 40))]
+    batch = capi.Batch(len(ens))
+    sims = [capi.Simulation(*e, weights=golden_weights) for e in ens]
+    for s in sims:
+        batch.add(s)
+    batch.run(4)
+    for sim, e in zip(sims, ens):
+        steps = e[2].num_timesteps
+        assert sim.next_step == steps
+        np.testing.assert_array_equal(sim.state(), solo(*e, golden_weights, steps)[0])
+    batch.close()
+    for s in sims:
+        s.close()
