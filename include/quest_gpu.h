@@ -27,8 +27,8 @@
  *    either); different handles are independent.
  *  - The library allocates its device memory in qg_create and frees it in
  *    qg_destroy; no call in between allocates device memory (the first
- *    evaluate or history copy of a handle allocates its small pinned host
- *    staging buffer).  The memory
+ *    evaluate, history copy or small recorded run of a handle takes a small
+ *    pinned host buffer).  The memory
  *    comes from a stream-ordered pool per device that keeps freed blocks (up
  *    to half the device's memory) for later handles, so qg_destroy does not
  *    synchronise the device; an allocation that does not fit first returns
