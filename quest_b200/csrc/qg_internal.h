@@ -202,6 +202,22 @@ struct StepArgs {
   PCW w;
 };
 
+// A dot's run of the mid list: its entries' partners and delays, its
+// coefficients (q + 1 per entry) and how many of those there are.  Offsets into
+// the lists are ints, but an offset times q + 1 need not fit one: a group of
+// 16 400 dots coupled to one another has 2^28 entries, whose coefficients at
+// q = 7 are 2^31.
+struct MidRow {
+  const int *idx, *delay;
+  const double2 *coef;
+  int taps;
+};
+__host__ __device__ inline MidRow mid_row(const StepArgs &a, int dot)
+{
+  const int e0 = a.mid_ptr[dot], e1 = a.mid_ptr[dot + 1], q1 = a.q + 1;
+  return MidRow{a.mid_idx + e0, a.mid_delay + e0, a.mid_coef + (long long)e0 * q1, (e1 - e0) * q1};
+}
+
 // Scratch of the allocation-free evaluation (qg_history_evaluate_noalloc):
 // a static device array in qg_far.cu, at most kNoAllocMaxDots padded dots.
 constexpr int kNoAllocMaxDots = 4096;

@@ -1132,30 +1132,30 @@ constexpr int kPastFlight = 8;
 __device__ __forceinline__ double2 group_past(const StepArgs &a, int idx, int t)
 {
   const int q1 = a.q + 1, lane = threadIdx.x & 31, tslot = ring_slot(t, a.W);
-  const int m0 = a.mid_ptr[idx] * q1, m1 = a.mid_ptr[idx + 1] * q1;
+  const MidRow m = mid_row(a, idx);
   double2 f[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-  for(int j0 = m0 + lane; j0 < m1; j0 += 32 * kPastFlight) {
+  for(int j0 = lane; j0 < m.taps; j0 += 32 * kPastFlight) {
     // no branch between the loads: a product past the end repeats the last
     // one, and is not added
     int e[kPastFlight], d[kPastFlight], b[kPastFlight];
     double2 v[kPastFlight], c[kPastFlight];
 #pragma unroll
     for(int u = 0; u < kPastFlight; ++u) {
-      e[u] = min(j0 + 32 * u, m1 - 1) / q1;
-      d[u] = __ldg(a.mid_delay + e[u]);
-      b[u] = __ldg(a.mid_idx + e[u]);
+      e[u] = min(j0 + 32 * u, m.taps - 1) / q1;
+      d[u] = __ldg(m.delay + e[u]);
+      b[u] = __ldg(m.idx + e[u]);
     }
 #pragma unroll
     for(int u = 0; u < kPastFlight; ++u) {
-      const int j = min(j0 + 32 * u, m1 - 1), back = d[u] + (j - e[u] * q1);
+      const int j = min(j0 + 32 * u, m.taps - 1), back = d[u] + (j - e[u] * q1);
       const int slot = tslot - back + (tslot < back ? a.W : 0);
       v[u] = __ldcg(a.ring + (long long)b[u] * a.stride + slot);
-      c[u] = __ldg(a.mid_coef + j);
+      c[u] = __ldg(m.coef + j);
     }
 #pragma unroll
     for(int u = 0; u < kPastFlight; ++u) {
       const int j = j0 + 32 * u, back = d[u] + (j - e[u] * q1);
-      if(j < m1 && t - back >= -kWindow && back >= 1) {
+      if(j < m.taps && t - back >= -kWindow && back >= 1) {
         const double2 p = cmul(prefactor(v[u], a.frame), c[u]);
         f[u & 1].x += p.x;
         f[u & 1].y += p.y;
