@@ -127,7 +127,9 @@ qg_status qg_pc_weights(int n_lambda, int n_time, double radius, qg_weights *out
  * coefficient table (history_interaction.cpp:5-45), PulseInteraction, the
  * History array initialised as main.cpp:30-36 does (rho = (1,0) for
  * t <= 0), and the Integrator's weights.  weights == NULL uses
- * qg_pc_weights(18, 22, 3.15), the values main.cpp:48-49 hard-codes. */
+ * qg_pc_weights(18, 22, 3.15), the values main.cpp:48-49 hard-codes.
+ * QG_ERR_UNSUPPORTED where 2^30 or more pairs have a floor delay below 16 (the
+ * step kernels' lists are addressed by 32-bit entry). */
 qg_status qg_create(const qg_dot *dots, int n, const qg_pulse *pulse,
                     const qg_params *params, const qg_weights *weights,
                     qg_handle **out);

@@ -575,6 +575,9 @@ static qg_status build_lists(qg_handle *h, const TableArgs &ta)
     QG_CUDA(cudaGetLastError());
     QG_CUDA(cudaMemcpyAsync(&cnt, h->d_u64 + 2, sizeof cnt, cudaMemcpyDeviceToHost, h->stream));
     QG_CUDA(cudaStreamSynchronize(h->stream));
+    if(!mid_list_fits(cnt))
+      return qg_fail(QG_ERR_UNSUPPORTED, "qg_create: %llu pairs with a delay below %d steps; their lists hold at "
+                     "most 2^30 - 1", cnt, kTimeBlock);
   }
   h->mid_pairs = (long long)cnt;
   launch_pair_list_coef(ta, h->q, d_pairs, (long long)cnt, d_mc, h->stream);

@@ -218,6 +218,10 @@ __host__ __device__ inline MidRow mid_row(const StepArgs &a, int dot)
   return MidRow{a.mid_idx + e0, a.mid_delay + e0, a.mid_coef + (long long)e0 * q1, (e1 - e0) * q1};
 }
 
+// Whether the lists of `pairs` pairs with floor delay < K, an entry for each
+// dot of a pair, can be addressed: their offsets are ints.
+inline bool mid_list_fits(unsigned long long pairs) { return pairs <= 0x7fffffffULL / 2; }
+
 // Scratch of the allocation-free evaluation (qg_history_evaluate_noalloc):
 // a static device array in qg_far.cu, at most kNoAllocMaxDots padded dots.
 constexpr int kNoAllocMaxDots = 4096;

@@ -1,6 +1,7 @@
 // The offsets a dot's run of the mid list starts at (mid_row), around 2^31
-// coefficients: addresses compared as integers, nothing is read but the two
-// list bounds.  Exit status 1 on any mismatch.
+// coefficients (addresses compared as integers, nothing is read but the two
+// list bounds), and the pair counts whose lists the library builds
+// (mid_list_fits).  Exit status 1 on any mismatch.
 #include <cstdint>
 #include <cstdio>
 
@@ -27,6 +28,13 @@ int main()
                       r.taps == 5 * (q + 1);
       if(!ok) std::printf("mismatch: q %d, entries up to %d\n", q, last), ++bad;
     }
+  // 2^30 - 1 pairs are 2^31 - 2 entries, one pair more is past an int; a count
+  // whose double wraps in 32 or 64 bits is refused like any other
+  const unsigned long long p30 = 1ULL << 30;
+  if(!qg::mid_list_fits(0) || !qg::mid_list_fits(p30 - 1)) std::printf("mismatch: refused a list that fits\n"), ++bad;
+  const unsigned long long many[] = {p30, 2 * p30, 2 * p30 + 5, 4 * p30, 1ULL << 63};
+  for(unsigned long long p : many)
+    if(qg::mid_list_fits(p)) std::printf("mismatch: accepted %llu pairs\n", p), ++bad;
   std::printf("mismatches %d\n", bad);
   return bad != 0;
 }
