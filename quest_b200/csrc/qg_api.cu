@@ -133,6 +133,9 @@ struct qg_handle_s {
   // the ring slots of steps before -22 hold the zeros of the last reset: no
   // caller has written history since
   bool ring_clean = false;
+  // a call that writes history was captured: its replays write the ring
+  // without the host's knowledge, so no later reset counts as clean
+  bool ring_replayed = false;
   bool tune_pending = false;  // the far-kernel autotuner runs at the first qg_run
   bool profile = false;
   // first bad step as the last batch run read it (qg_bad_step answers from it
@@ -1321,7 +1324,8 @@ static void record_event(qg_handle *h, cudaEvent_t e)
 static int far_form(const qg_handle *h, int t0)
 {
   if(t0 >= h->max_delay + h->q - kWindow) return kFormPlain;
-  return h->far_early && h->ring_clean && !h->far_nonfinite ? kFormPlain : kFormAny;
+  const bool zeros = h->ring_clean && !h->ring_replayed;
+  return h->far_early && zeros && !h->far_nonfinite ? kFormPlain : kFormAny;
 }
 
 static void enqueue_far(qg_handle *h, int t0, bool at_boundary, cudaEvent_t ea, cudaEvent_t eb, int form)
@@ -2385,6 +2389,9 @@ extern "C" qg_status qg_history_evaluate_noalloc(qg_handle *h, int step, const d
   cudaStream_t s = stream ? (cudaStream_t)stream : h->stream;
   StepArgs a = h->step_args(true);
   if(d_rho01_step) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    QG_CUDA(cudaStreamIsCapturing(s, &capture));
+    if(capture != cudaStreamCaptureStatusNone) h->ring_replayed = true;
     h->ring_clean = false;
     launch_ring_write(a, step, (const double2 *)d_rho01_step, s);
     launch_ring32_rebuild(a, s);

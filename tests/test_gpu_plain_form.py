@@ -1,0 +1,81 @@
+"""The far kernel's plain form in the blocks where some windows start before
+step -22: it reads the samples of those steps as the zeros the ring was reset
+to, and is taken only where that changes no bit.  Whatever the history holds,
+a run gives what it gives with "far_early" 0,
+where each such sample is skipped."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from quest_b200 import capi, inputs as I
+
+pytestmark = pytest.mark.gpu
+
+
+def workload(n, frame, q, steps):
+    wl = I.plain_table(seed=4, n=n, steps=steps, pulse_delay=0.05)
+    wl.dots[:, 6:9] *= 0.1
+    wl.constants.frame = frame
+    wl.constants.interpolation_order = q
+    return wl
+
+
+@pytest.mark.parametrize("replay_before_reset", [False, True])
+def test_a_replayed_evaluation_writes_the_ring(golden_weights, replay_before_reset):
+    """qg_history_evaluate_noalloc captured once and replayed after a reset:
+    its iterate goes into a slot that the first blocks' windows share with a
+    step before -22, and the run is the one without it."""
+    import torch
+
+    wl = workload(300, 0, 5, 400)
+    with capi.Simulation(wl.dots, wl.pulse, wl.constants, weights=golden_weights, coef_mode=capi.COEF_TABLE) as sim:
+        clean = sim.run(96)
+        sim.set_option("reset", 1)
+        step = sim.info()["ring_depth"] - 40  # step -40's slot
+        assert 112 < step < 400
+        d_in = torch.full((sim.n,), 1 + 1j, dtype=torch.complex128, device="cuda")
+        d_out = torch.empty((sim.n,), dtype=torch.complex128, device="cuda")
+
+        def evaluate(iterate, stream):
+            rc = capi.lib().qg_history_evaluate_noalloc(
+                sim.h, step, ctypes.c_void_p(d_in.data_ptr()) if iterate else None,
+                ctypes.c_void_p(d_out.data_ptr()), ctypes.c_void_p(stream.cuda_stream))
+            assert rc == capi.QG_OK, capi.lib().qg_last_error().decode()
+
+        s = torch.cuda.Stream()
+        evaluate(False, s)  # the first call looks the scratch's address up, before the capture
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            evaluate(True, torch.cuda.current_stream())
+        if replay_before_reset:
+            g.replay()
+            torch.cuda.synchronize()
+        sim.set_option("reset", 1)
+        g.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(sim.get_history(step, 1)[0], np.full(sim.n, 1 + 1j))
+        got = sim.run(96)
+    np.testing.assert_array_equal(clean, got)
+
+
+@pytest.mark.parametrize("mode", [capi.COEF_TABLE, capi.COEF_ON_THE_FLY])
+@pytest.mark.parametrize("precision", [capi.PREC_FP64, capi.PREC_MIXED])
+@pytest.mark.parametrize("frame,q", [(0, 5), (1, 3)])
+def test_both_forms_give_the_same_bits(golden_weights, mode, precision, frame, q):
+    """All the blocks of a run from the ground state past the largest delay
+    (about 300 steps), through a checkpoint taken among them."""
+    wl = workload(700, frame, q, 352)
+    outs = []
+    for early in (1, 0):
+        with capi.Simulation(wl.dots, wl.pulse, wl.constants, weights=golden_weights, precision=precision,
+                             coef_mode=mode) as sim:
+            sim.set_option("far_early", early)
+            first = sim.run(40)
+            data = sim.checkpoint()
+            sim.run(24)
+            sim.restore(data)
+            outs.append(np.concatenate([first, sim.run(312)]))
+    assert np.abs(outs[0][..., 1]).max() > 1e-8
+    np.testing.assert_array_equal(outs[0], outs[1])
