@@ -12,8 +12,9 @@ namespace qg {
 
 // ---- accumulators --------------------------------------------------------------
 // One lane's K far-field sums.  Rotating frame: complex taps on complex
-// samples.  Lab frame (prefactor 2 Re rho01, real taps): real products only,
-// the imaginary parts being exact zeros.
+// samples.  Lab frame (prefactor 2 Re rho01, real taps): real products only.
+// The imaginary part of a complex product of them is zero, or NaN where a
+// factor is not finite (and the real part is not either): v * 0.
 template <bool LAB, int K>
 struct FarAcc;
 
@@ -66,7 +67,7 @@ struct FarAcc<true, K> {
 #pragma unroll
     for(int k = (m - Q > 0 ? m - Q : 0); k <= (m < K - 1 ? m : K - 1); ++k) v[k] = fma(c[k + Q - m], x, v[k]);
   }
-  __device__ __forceinline__ double2 out(int k) const { return make_double2(v[k], 0.0); }
+  __device__ __forceinline__ double2 out(int k) const { return make_double2(v[k], v[k] * 0.0); }
 };
 
 // Packed FP32 pairs (Blackwell fma.rn.f32x2 / add.rn.f32x2): one instruction
@@ -177,7 +178,11 @@ struct MixedAcc<true, Q, K> {
   __device__ __forceinline__ void add(float2 d) { u += 2.f * d.x; }
   __device__ __forceinline__ float absolute(float2 w0) const { return 2.f * w0.x + u; }
   __device__ __forceinline__ void mac(int k, int i, float w) { a[k] = fmaf(cx[i], w, a[k]); }
-  __device__ __forceinline__ double2 out(int k) const { return make_double2((double)a[k] + (double)base, 0.0); }
+  __device__ __forceinline__ double2 out(int k) const
+  {
+    const double v = (double)a[k] + (double)base;
+    return make_double2(v, v * 0.0);
+  }
 };
 
 // ---- windows read from the ring ------------------------------------------------
