@@ -935,6 +935,26 @@ static qg_status order_for_near_groups(qg_handle *h, const qg_dot *dots, const s
   return QG_OK;
 }
 
+// Whether no tap of a far pair computed on the fly, nor anything it is formed
+// from (pair_coef_otf, pair_coef_otf_mixed), can overflow: `dip` bounds the
+// dipoles' components, `reach` every distance.  A far pair is K c dt apart or
+// further.  The bounds leave room for the weights' polynomials and node sums,
+// a factor of 2^20 in FP32 and, with reciprocals of fractions down to 2^-49
+// squared in the FP64 form, 2^100 there.
+static bool otf_taps_finite(const qg_params &p, double dip, double reach, bool mixed)
+{
+  const double c = std::fabs(p.c0), idt = std::fabs(1 / p.dt), om = std::fabs(p.laser_frequency);
+  const double A = std::fabs(p.mu0 / p.hbar), ir = idt / (kTimeBlock * c), dd = 12 * dip * dip;
+  const double G0 = dd * c * c * ir * ir * ir, G1 = dd * c * ir * ir, G2 = dd * ir;
+  const double a0 = G0 + om * G1 + om * om * G2, a1 = (G1 + 2 * om * G2) * idt, a2 = 2 * G2 * idt * idt;
+  const double all[] = {dd * reach * reach, reach * reach, c, dd * c * c, ir * ir * ir, om * om, 2 * idt * idt,
+                        a0, a1, a2, A, A * G0, A * G1, A * G2, A * a0, A * a1, A * a2, om * reach / c};
+  const double limit = mixed ? 0x1p108 : 0x1p924;
+  for(double v : all)
+    if(!(v < limit)) return false;
+  return true;
+}
+
 static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, const qg_params *p,
                              const qg_weights *weights, qg_handle *h)
 {
@@ -1087,11 +1107,21 @@ static qg_status create_impl(const qg_dot *dots, int n, const qg_pulse *pulse, c
   h->near_pairs = (long long)nn[0];  // on the fly: counted from the mid list below
   h->mid_pairs = (long long)nn[1];
   h->far_nonfinite = nn[3] > 0;
-  if(h->otf) {
-    // on the fly nothing was computed yet: any non-finite input counts too
-    bool fin = std::isfinite(p->mu0 / p->hbar) && std::isfinite(p->laser_frequency);
+  if(h->otf || h->tune_coef) {
+    // on the fly nothing was computed yet: any non-finite input counts too, and
+    // any from which a tap could overflow
+    bool fin = true;
+    double dip = 0, lo[3], hi[3];
+    for(int k = 0; k < 3; ++k) lo[k] = hi[k] = dots[0].pos[k];
     for(int i = 0; i < n && fin; ++i)
-      for(int k = 0; k < 3; ++k) fin = fin && std::isfinite(dots[i].dip[k]) && std::isfinite(dots[i].pos[k]);
+      for(int k = 0; k < 3; ++k) {
+        fin = fin && std::isfinite(dots[i].dip[k]) && std::isfinite(dots[i].pos[k]);
+        dip = std::max(dip, std::fabs(dots[i].dip[k]));
+        lo[k] = std::min(lo[k], dots[i].pos[k]);
+        hi[k] = std::max(hi[k], dots[i].pos[k]);
+      }
+    const double reach = (hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2]);
+    fin = fin && otf_taps_finite(*p, dip, reach, h->mixed);
     h->far_nonfinite = h->far_nonfinite || !fin;
   }
 

@@ -82,31 +82,34 @@ __global__ void __launch_bounds__(128) table_build_kernel(TableArgs a)
   const int fd = pair_coef_ref<Q>(ps, po, ds, dob, a.cp, coef);
   *d1 = fd;
   *d2 = fd;
+  bool fin = true;  // the coefficients as they are held
   if(MIXED) {
     double2 sum = make_double2(0.0, 0.0);
 #pragma unroll
     for(int i = 0; i <= Q; ++i) {
       const float2 v = make_float2((float)coef[i].x, (float)coef[i].y);
       f1[(long long)i * kTilePairs] = f2[(long long)i * kTilePairs] = v;
+      fin = fin && isfinite(v.x) && isfinite(v.y);
       sum.x += coef[i].x;
       sum.y += coef[i].y;
     }
-    f1[(long long)(Q + 1) * kTilePairs] = f2[(long long)(Q + 1) * kTilePairs] = make_float2((float)sum.x, (float)sum.y);
+    const float2 v = make_float2((float)sum.x, (float)sum.y);
+    f1[(long long)(Q + 1) * kTilePairs] = f2[(long long)(Q + 1) * kTilePairs] = v;
+    fin = fin && isfinite(v.x) && isfinite(v.y);
   } else {
 #pragma unroll
-    for(int i = 0; i <= Q; ++i) c1[(long long)i * kTilePairs] = c2[(long long)i * kTilePairs] = coef[i];
+    for(int i = 0; i <= Q; ++i) {
+      c1[(long long)i * kTilePairs] = c2[(long long)i * kTilePairs] = coef[i];
+      fin = fin && isfinite(coef[i].x) && isfinite(coef[i].y);
+    }
   }
   atomicMax(a.max_delay, fd);
   if(fd == 0) atomicAdd(a.near_count, 1ULL);
   if(fd < kTimeBlock) atomicAdd(a.near_count + 1, 1ULL);
-  if(fd >= kTimeBlock) {
-    // far pairs with a non-finite coefficient (an integer delay): the far
-    // kernels' plain form is not used for the first blocks of such a table
-    bool fin = true;
-#pragma unroll
-    for(int i = 0; i <= Q; ++i) fin = fin && isfinite(coef[i].x) && isfinite(coef[i].y);
-    if(!fin) atomicAdd(a.near_count + 3, 1ULL);
-  }
+  // far pairs with a non-finite coefficient (an integer delay, an overflow):
+  // the far kernels' plain form is not used for the first blocks of such a
+  // table
+  if(fd >= kTimeBlock && !fin) atomicAdd(a.near_count + 3, 1ULL);
 }
 
 template <bool MIXED>

@@ -1,13 +1,14 @@
 """The far kernel's plain form in the blocks where some windows start before
 step -22: it reads the samples of those steps as the zeros the ring was reset
-to, and is taken only where that changes no bit.  Whatever the history holds,
-a run gives what it gives with "far_early" 0,
+to, and is taken only where that changes no bit.  Whatever the history holds
+and whatever the coefficients, a run gives what it gives with "far_early" 0,
 where each such sample is skipped."""
 import ctypes
 
 import numpy as np
 import pytest
 
+from oracle import oracle as O
 from quest_b200 import capi, inputs as I
 
 pytestmark = pytest.mark.gpu
@@ -58,6 +59,28 @@ def test_a_replayed_evaluation_writes_the_ring(golden_weights, replay_before_res
         np.testing.assert_array_equal(sim.get_history(step, 1)[0], np.full(sim.n, 1 + 1j))
         got = sim.run(96)
     np.testing.assert_array_equal(clean, got)
+
+
+@pytest.mark.parametrize("precision,mode,scale", [
+    (capi.PREC_FP64, capi.COEF_TABLE, 1e160), (capi.PREC_FP64, capi.COEF_ON_THE_FLY, 1e160),
+    (capi.PREC_MIXED, capi.COEF_TABLE, 1e20), (capi.PREC_MIXED, capi.COEF_ON_THE_FLY, 1e20)])
+@pytest.mark.parametrize("frame", [0, 1])
+def test_coefficients_that_overflow(golden_weights, oracle_weights, precision, mode, scale, frame):
+    """Dipoles whose coefficients are infinite in the precision they are held
+    in: two dots 30.5 steps apart, no pulse.  Step 8 is the first with a tap
+    that reads step -22, where the product with zero is NaN."""
+    c = I.Constants(c0=1.0, dt=0.125, num_timesteps=40, frame=frame)
+    dots = np.array([[0.0, 0, 0, 200, 10, 10, 0, 0, scale],
+                     [30.5 * 0.125, 0, 0, 200, 10, 10, 0, 0, scale]])
+    pulse = I.make_pulse(amplitude=0.0)
+    if precision == capi.PREC_FP64:
+        assert O.run_faithful(dots, pulse, c, oracle_weights, 40)[1] == 8
+    for early in (1, 0):
+        with capi.Simulation(dots, pulse, c, weights=golden_weights, precision=precision, coef_mode=mode) as sim:
+            sim.set_option("far_early", early)
+            with pytest.raises(capi.NonFiniteError) as e:
+                sim.run(40)
+        assert e.value.step == 8, early
 
 
 @pytest.mark.parametrize("mode", [capi.COEF_TABLE, capi.COEF_ON_THE_FLY])
