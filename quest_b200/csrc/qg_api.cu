@@ -798,8 +798,8 @@ static qg_status build_lists(qg_handle *h, const TableArgs &ta)
   return QG_OK;
 }
 
-// The step kernels' flags start alike (a launch that gave up a wait leaves them
-// apart).
+// The step kernels' flags start alike (a launch that gave up a wait, or in which
+// a block did not post, leaves them apart).
 static qg_status clear_flags(qg_handle *h)
 {
   QG_CUDA(cudaMemsetAsync(h->d_flags, 0, sizeof(unsigned) * (size_t)std::max(h->step_blocks, 1) * kFlagStride,
@@ -2570,6 +2570,9 @@ extern "C" qg_status qg_set_option(qg_handle *h, const char *key, int value)
       if(value < -1 || value >= std::max(h->step_blocks, 1))
         return qg_fail(QG_ERR_INVALID_ARG, "qg_set_option: test_skip_post in -1 .. %d", h->step_blocks - 1);
       h->skip_post = value;
+      // a block that skipped posts stands behind the others
+      QG_CUDA(cudaSetDevice(h->device));
+      QG_TRY(clear_flags(h));
     } else if(!std::strcmp(key, "far_group")) {
       if(h->otf || value < 1 || (h->nT > 512 && value < far_group(h->mixed, h->nT)))
         return qg_fail(QG_ERR_INVALID_ARG, "qg_set_option: far_group %d not available (table handles, "
