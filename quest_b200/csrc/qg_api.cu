@@ -155,9 +155,9 @@ struct qg_handle_s {
   int pair_launches = 0, step_launches = 0;
   cudaEvent_t ev_chunk[2] = {nullptr, nullptr}, ev_copy[2] = {nullptr, nullptr};
 
-  // `groups`: source tiles per group; `parts` per group (0: far_parts' cut)
-  FarArgs far_args(const int *d_t0, int *far_t0_out) const { return far_args(d_t0, far_t0_out, group, 0); }
-  FarArgs far_args(const int *d_t0, int *far_t0_out, int groups, int parts) const
+  // `groups`: source tiles per group
+  FarArgs far_args(const int *d_t0, int *far_t0_out) const { return far_args(d_t0, far_t0_out, group); }
+  FarArgs far_args(const int *d_t0, int *far_t0_out, int groups) const
   {
     FarArgs s{};
     s.delay = d_delay;
@@ -177,7 +177,7 @@ struct qg_handle_s {
     s.frame = params.frame;
     groups = std::min(groups, nT);  // a larger group holds the same sources
     s.group = groups;
-    s.parts = parts > 0 ? parts : far_parts(nT, groups);
+    s.parts = far_parts(nT, groups);
     s.unit = (groups * kTile + s.parts - 1) / s.parts;
     s.nP = (nT + groups - 1) / groups * s.parts;
     s.d_t0 = d_t0;
@@ -2429,8 +2429,8 @@ extern "C" qg_status qg_history_evaluate_noalloc(qg_handle *h, int step, const d
     h->far_block = -0x7fffffff;
   }
   launch_set_int(sc.ints + 0, step, s);
-  // the fixed scratch holds the partials of this group size, uncut
-  FarArgs fa = h->far_args(sc.ints + 0, sc.ints + 1, kTileGroup, 1);
+  // the fixed scratch holds the partials of this group size, cut as always
+  FarArgs fa = h->far_args(sc.ints + 0, sc.ints + 1, kTileGroup);
   fa.partial = sc.partial;
   fa.field = sc.field;
   launch_far_step1(fa, s);

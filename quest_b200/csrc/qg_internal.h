@@ -224,13 +224,15 @@ inline bool mid_list_fits(unsigned long long pairs) { return pairs <= 0x7fffffff
 
 // Scratch of the allocation-free evaluation (qg_history_evaluate_noalloc):
 // a static device array in qg_far.cu, at most kNoAllocMaxDots padded dots.
+// Uncut, the partials are kNoAllocMaxGroups x n_pad at most; where far_parts
+// cuts the groups there are 1776 tasks at most, 1776 x 32 values.
 constexpr int kNoAllocMaxDots = 4096;
 constexpr int kNoAllocMaxTiles = kNoAllocMaxDots / kTile;
 constexpr int kNoAllocMaxGroups = (kNoAllocMaxTiles + kTileGroup - 1) / kTileGroup;
 constexpr size_t kNoAllocScratchTotal = 16ull * kNoAllocMaxGroups * kNoAllocMaxDots + 16ull * kNoAllocMaxDots +
                                         256;
 struct NoAllocScratch {
-  double2 *partial;    // [kNoAllocMaxGroups][n_pad]
+  double2 *partial;    // [nP][n_pad], room for kNoAllocMaxGroups * kNoAllocMaxDots
   double2 *field;      // [n_pad]
   int *ints;           // [0] step, [1] far_t0 written by the kernel
 };
