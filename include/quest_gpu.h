@@ -259,8 +259,8 @@ qg_status qg_batch_set_option(qg_batch *b, const char *key, int value);
  * group tuned for each size class, 0 = members keep their own),
  * "tuned_far_us" (the far launch's time the batch's autotuner measured for
  * its choice, microseconds; 0 if it did not run).  The autotuner times the
- * far launch at the batch's first qg_batch_run; "autotune" (1) asks for it
- * again at the next run. */
+ * far launch at the batch's first qg_batch_run, unless "far_packed" or
+ * "far_gmajor" was set; "autotune" (1) asks for it again at the next run. */
 qg_status qg_batch_get_option(const qg_batch *b, const char *key, int *value);
 /* Device time in milliseconds of the batch's far-pair launches and step
  * launches (each nullable), accumulated while "profile" is on. */

@@ -2092,10 +2092,12 @@ extern "C" qg_status qg_batch_set_option(qg_batch *b, const char *key, int value
   }
   if(!std::strcmp(key, "far_packed")) {
     b->far_packed = value != 0;
+    b->tune_pending = false;  // an explicit choice is kept
     return QG_OK;
   }
   if(!std::strcmp(key, "far_gmajor")) {
     b->far_gmajor = value != 0;
+    b->tune_pending = false;  // an explicit choice is kept
     return QG_OK;
   }
   if(!std::strcmp(key, "autotune")) {
