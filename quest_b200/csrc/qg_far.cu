@@ -285,40 +285,25 @@ void launch_far_reduce(const FarArgs &a, int steps, void *stream)
 }
 
 // ---- launches ----------------------------------------------------------------------
-// The stages' dynamic shared memory (28 KB a block at q = 5) is opted in once
-// per function and device.
 template <int Q, bool MIXED>
 constexpr size_t far_smem_bytes()
 {
   return MIXED ? 0 : kFarWarps * sizeof(FarStage<Q>);
 }
-
-template <class Fn>
-static void far_smem_optin(Fn *fn, size_t bytes, bool (&done)[64])
-{
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if(bytes == 0 || (dev < 64 && done[dev])) return;
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if(dev < 64) done[dev] = true;
-}
+// 28 KB a block at q = 5, 36 KB at the largest order: no opt-in needed
+static_assert(far_smem_bytes<kMaxOrder, false>() <= 48 << 10, "dynamic shared memory without an opt-in");
 
 template <int Q, bool LAB, bool MIXED, int FORM>
 static void launch_far_q(const FarArgs &a, cudaStream_t s)
 {
-  static bool done[64] = {};
-  constexpr size_t smem = far_smem_bytes<Q, MIXED>();
-  far_smem_optin(far_kernel<Q, LAB, MIXED, FORM>, smem, done);
-  far_kernel<Q, LAB, MIXED, FORM><<<far_blocks(a), 32 * kFarWarps, smem, s>>>(a);
+  far_kernel<Q, LAB, MIXED, FORM><<<far_blocks(a), 32 * kFarWarps, far_smem_bytes<Q, MIXED>(), s>>>(a);
 }
 
 template <int Q, bool LAB, bool MIXED, int FORM>
 static void launch_far_batch_q(const FarArgs *args, const int *task_off, int n_ens, int blocks, cudaStream_t s)
 {
-  static bool done[64] = {};
-  constexpr size_t smem = far_smem_bytes<Q, MIXED>();
-  far_smem_optin(far_batch_kernel<Q, LAB, MIXED, FORM>, smem, done);
-  far_batch_kernel<Q, LAB, MIXED, FORM><<<blocks, 32 * kFarWarps, smem, s>>>(args, task_off, n_ens);
+  far_batch_kernel<Q, LAB, MIXED, FORM>
+      <<<blocks, 32 * kFarWarps, far_smem_bytes<Q, MIXED>(), s>>>(args, task_off, n_ens);
 }
 
 // calls f<q>() for the run-time order
