@@ -349,13 +349,15 @@ qg_status qg_kernel_time(qg_handle *h, int reset, double *pair_ms, int *pair_lau
  * "block_step" (1 = the K steps of a block in one cooperative launch, the
  *   default where every 32-dot block fits on the device at once; 0 = one
  *   launch per step; same results),
- * "wait_limit" (polls the step-block kernel makes on a partner block's step
- *   count before it gives up; 0 = the default, about a second.  A wait that
- *   runs out ends the launch: qg_run returns QG_ERR_CUDA "timed out" and the
- *   handle needs "reset" or a checkpoint load before it runs again),
- * "test_skip_post" (failure-detection tests only: the index of a 32-dot block
- *   that never posts its finished steps, so that its partners' waits run
- *   out; -1 = none, the default),
+ * "wait_limit" (polls the step kernels make on other blocks before they give
+ *   up: the step-block kernel on a partner block's step count, the general
+ *   form's grid (more than 256 dots) on the blocks it exchanges iterates with;
+ *   0 = the default, about a second.  A wait that runs out ends the launch:
+ *   qg_run returns QG_ERR_CUDA "timed out" and the handle needs "reset" or a
+ *   checkpoint load before it runs again),
+ * "test_skip_post" (failure-detection tests only: the index of a block of one
+ *   of those launches that never posts, so that the others' waits run out;
+ *   -1 = none, the default; no effect where blocks do not wait by polling),
  * "reset" (restart the history at step 0, main.cpp:30-36). */
 qg_status qg_set_option(qg_handle *h, const char *key, int value);
 

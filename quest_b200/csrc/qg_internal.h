@@ -193,9 +193,10 @@ struct StepArgs {
   int *d_next;           // first step of the next far block (set by the last
                          // step kernel of a block, read by the far kernel)
   int *d_bad;
-  // step-block kernel: polls per wait on a partner block before it gives up
-  // (0: the default, about a second), and a block that never posts its steps
-  // (-1: none; set only by failure-detection tests, so that waits run out)
+  // step-block kernel and the general form's grid: polls per wait on other
+  // blocks before it gives up (0: the default, about a second), and a block
+  // that never posts (-1: none; set only by failure-detection tests, so that
+  // waits run out)
   int spin_limit;
   int skip_post_block;
   int blk_lo;  // first 32-dot block of the per-step launch (a shard's range)

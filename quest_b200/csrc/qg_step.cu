@@ -1290,7 +1290,7 @@ __global__ void __launch_bounds__(kGroupThreads) step_group_kernel(StepArgs a, i
       } else {
         __syncthreads();
         if(threadIdx.x == 0) {
-          post_step(counter);
+          if((int)blockIdx.x != a.skip_post_block) post_step(counter);
           const int limit = a.spin_limit > 0 ? a.spin_limit : kGridSpins;
           int spins = 0;
           while(ld_acquire(counter) < (epoch + 1) * nb) {
