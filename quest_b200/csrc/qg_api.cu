@@ -186,16 +186,7 @@ struct qg_handle_s {
     s.pos = d_pos;
     s.dip = d_dip;
     s.user = d_user;
-    s.oc.c0dt = params.c0 * params.dt;
-    s.oc.inv_c0dt = 1.0 / s.oc.c0dt;
-    s.oc.c0 = params.c0;
-    s.oc.c0_sq = params.c0 * params.c0;
-    s.oc.A = params.mu0 / (4 * M_PI * params.hbar);
-    s.oc.inv_dt = 1.0 / params.dt;
-    s.oc.inv_dt2 = s.oc.inv_dt * s.oc.inv_dt;
-    s.oc.om = params.laser_frequency;
-    s.oc.om_sq = params.laser_frequency * params.laser_frequency;
-    s.oc.half_turns = params.laser_frequency / (M_PI * params.c0);
+    s.oc = otf_const(params);
     s.tile_lo = shard_world > 1 ? blk_lo : 0;  // 32-dot blocks are the 32-dot target tiles
     s.tile_n = shard_world > 1 ? blk_hi - blk_lo : 0;
     return s;

@@ -168,14 +168,31 @@ __device__ __forceinline__ double div_by(double x, double t, double y)
   return r == 0.0 ? q0 : fma(r, y, q0);
 }
 
-// 1 / x to about an ulp: the hardware's approximation (20 bits or more) and
-// one third-order Newton step, y (1 + e + e^2) with e = 1 - x y.
+// 1 / x: the hardware's approximation y, whose error is 2^-20 or less, and one
+// step of the third-order hyperpower iteration (M. Altman, Pacific J. Math. 10,
+// 1960), y (1 + e + e^2) with e = 1 - x y, which leaves e^3.  With the last
+// multiply-add's rounding the error is 2^-53 (1 + 2^-6) at most.
+__device__ __forceinline__ double rcp_refine(double x, double y)
+{
+  const double e = fma(-x, y, 1.0);
+  return fma(fma(e, e, e), y, y);
+}
 __device__ __forceinline__ double rcp_newton(double x)
 {
   double y;
+#ifdef __CUDA_ARCH__
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(fma(e, e, e), y, y);
+#else
+  y = (double)(float)(1.0 / x);  // host tests
+#endif
+  return rcp_refine(x, y);
+}
+
+// omega r / (pi c0), the phase in half turns, to half an ulp: the constant's
+// low part takes its rounding out.
+__device__ __forceinline__ double half_turns(double r, const OtfConst &o)
+{
+  return fma(r, o.half_turns, r * o.half_turns_low);
 }
 
 // Separation, floor delay and fraction of a pair, with the operations of
@@ -282,8 +299,8 @@ __device__ __forceinline__ void pair_coef_otf(const PairGeom &g, const double (&
     });
   } else {
     double sn, cs;
-    sincospi(g.nrm * o.half_turns, &sn, &cs);
-    const double sx = -(o.A * cs), sy = o.A * sn;  // s = -A e^{-i pi half_turns r}
+    sincospi(half_turns(g.nrm, o), &sn, &cs);
+    const double sx = -(o.A * cs), sy = o.A * sn;  // s = -A e^{-i omega r / c0}
     const double ar0 = fma(-o.om_sq, G2, G0), ai0 = o.om * G1;
     const double br0 = G1 * o.inv_dt, bi0 = 2.0 * (o.om * G2) * o.inv_dt;
     const double gr0 = G2 * o.inv_dt2;

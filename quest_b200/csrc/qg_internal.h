@@ -1,6 +1,7 @@
 // Internal declarations shared by the library's translation units.
 #pragma once
 
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 
@@ -45,8 +46,26 @@ struct OtfConst {
   double c0dt, inv_c0dt;  // c0 dt and its correctly rounded reciprocal
   double c0, c0_sq, A;    // A = mu0 / (4 pi hbar)
   double inv_dt, inv_dt2;
-  double om, om_sq, half_turns;  // half_turns = omega / (pi c0)
+  double om, om_sq;
+  double half_turns, half_turns_low;  // omega / (pi c0) in two parts
 };
+inline OtfConst otf_const(const qg_params &p)
+{
+  OtfConst o;
+  o.c0dt = p.c0 * p.dt;
+  o.inv_c0dt = 1.0 / o.c0dt;
+  o.c0 = p.c0;
+  o.c0_sq = p.c0 * p.c0;
+  o.A = p.mu0 / (4 * M_PI * p.hbar);
+  o.inv_dt = 1.0 / p.dt;
+  o.inv_dt2 = o.inv_dt * o.inv_dt;
+  o.om = p.laser_frequency;
+  o.om_sq = p.laser_frequency * p.laser_frequency;
+  const long double ht = p.laser_frequency / (3.141592653589793238462643L * p.c0);
+  o.half_turns = (double)ht;
+  o.half_turns_low = (double)(ht - o.half_turns);
+  return o;
+}
 
 struct PulseParams {
   double amp_pol[3];  // (amplitude / 2) * polarisation_k
