@@ -376,9 +376,12 @@ void launch_far(const FarArgs &a, void *stream)
 }
 
 // ---- one step ----------------------------------------------------------------------
-// The far-pair field of one step (evaluations), the table prefetched in
-// registers two sources ahead: its stream from HBM bounds it.
-template <int Q, bool LAB, bool MIXED>
+// The far-pair field of one step (evaluations).  The table's stream from HBM
+// bounds it, and each warp's entries are fetched AHEAD sources early in
+// registers: what is in flight is that times the warps an SM holds, and a
+// launch lasts whole waves of them (launch_far1_q chooses).  The same sums in
+// the same order either way.
+template <int Q, bool LAB, bool MIXED, int AHEAD>
 __global__ void __launch_bounds__(32 * kFarWarps) far_step1_kernel(FarArgs a)
 {
   const int lane = threadIdx.x & 31;
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(32 * kFarWarps) far_step1_kernel(FarArgs a)
   };
   std::conditional_t<MIXED, MixedAcc<LAB, Q, 1>, FarAcc<LAB, 1>> acc;
   acc.zero();
-  auto take = [&](Pair &x, int s) {
+  auto take = [&](const Pair &x, int s) {
     if(x.d >= kTimeBlock && x.d <= d_last) {
       const int tau0 = t0 - x.d - Q, slot = wrap_slot(tau0, a.W);
       if constexpr(MIXED)
@@ -420,23 +423,68 @@ __global__ void __launch_bounds__(32 * kFarWarps) far_step1_kernel(FarArgs a)
       else
         window_conv<Q, LAB, 1, kFormAny>(a.ring + (long long)s * a.stride, slot, tau0, x.c, acc);
     }
-    load(x, s + 2);
   };
-  Pair even, odd;
-  load(even, t.s0);
-  load(odd, t.s0 + 1);
+  Pair x[AHEAD];
+#pragma unroll
+  for(int u = 0; u < AHEAD; ++u) load(x[u], t.s0 + u);
 #pragma unroll 1
-  for(int s = t.s0; s < t.s1; s += 2) {
-    take(even, s);
-    take(odd, s + 1);
+  for(int s = t.s0; s < t.s1; s += AHEAD) {
+#pragma unroll
+    for(int u = 0; u < AHEAD; ++u) {
+      if constexpr(AHEAD == 2) {  // no third set of registers
+        take(x[u], s + u);
+        load(x[u], s + u + 2);
+      } else {
+        const Pair y = x[u];
+        load(x[u], s + u + AHEAD);
+        take(y, s + u);
+      }
+    }
   }
   store_partial<1>(a, t, acc);
+}
+
+// Blocks of the one-step kernel the device holds at once.
+template <int Q, bool LAB, bool MIXED, int AHEAD>
+static int far1_resident()
+{
+  static const int blocks = [] {
+    int dev = 0, sms = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, far_step1_kernel<Q, LAB, MIXED, AHEAD>, 32 * kFarWarps, 0);
+    return std::max(1, sms * per);
+  }();
+  return blocks;
+}
+
+// Mixed: one source ahead, at every size (microseconds an evaluation at order
+// 5, one against two ahead: 2048 dots 134 / 178, 4096 185 / 313, 5200 301 / 352).
+// FP64: three ahead while all blocks then run at once (2048 dots 147 / 172,
+// lab frame 143 / 178; past that 4096 dots 455 / 367), else two, or one where
+// its smaller register count saves a wave (3500 dots 247 / 335, 5200 488 / 557;
+// at equal waves, 4096 dots, 388 / 367).
+template <int Q, bool LAB, bool MIXED>
+static void launch_far1_q(const FarArgs &a, cudaStream_t s)
+{
+  const int blocks = far_blocks(a), threads = 32 * kFarWarps;
+  if constexpr(MIXED) {
+    far_step1_kernel<Q, LAB, true, 1><<<blocks, threads, 0, s>>>(a);
+  } else {
+    auto waves = [&](int resident) { return (blocks + resident - 1) / resident; };
+    if(blocks <= far1_resident<Q, LAB, false, 3>())
+      far_step1_kernel<Q, LAB, false, 3><<<blocks, threads, 0, s>>>(a);
+    else if(waves(far1_resident<Q, LAB, false, 1>()) < waves(far1_resident<Q, LAB, false, 2>()))
+      far_step1_kernel<Q, LAB, false, 1><<<blocks, threads, 0, s>>>(a);
+    else
+      far_step1_kernel<Q, LAB, false, 2><<<blocks, threads, 0, s>>>(a);
+  }
 }
 
 template <bool LAB, bool MIXED>
 static void launch_far1_frame(const FarArgs &a, cudaStream_t s)
 {
-#define CALL(QQ) far_step1_kernel<QQ, LAB, MIXED><<<far_blocks(a), 32 * kFarWarps, 0, s>>>(a)
+#define CALL(QQ) launch_far1_q<QQ, LAB, MIXED>(a, s)
   QG_BY_ORDER(a.q, CALL)
 #undef CALL
 }
