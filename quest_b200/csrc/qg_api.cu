@@ -84,7 +84,7 @@ struct qg_handle_s {
   int *d_new_ptr = nullptr, *d_new_idx = nullptr;  // taps reading step t-1
   double2 *d_new_coef = nullptr;
   bool lag = false;  // every delay-0/1 partner shares the dot's 32-dot block
-  // d_ints: 0 step, 1 done, 2 bad, 3 traj_t0, 4 eval_step, 5 max_delay,
+  // d_ints: 0 step, 1 ring written (checkpoint load), 2 bad, 3 traj_t0, 4 eval_step, 5 max_delay,
   //         6 far_t0 (run), 7 far block start request, 8 far_t0 (evaluate)
   int *d_ints = nullptr;
   unsigned long long *d_u64 = nullptr;
@@ -2252,19 +2252,6 @@ extern "C" qg_status qg_checkpoint_save(qg_handle *h, void *buf, size_t bytes)
   return QG_OK;
 }
 
-// Whether a saved ring's slots of steps from `next` on (which a run of fewer
-// than W - 22 steps shares with the steps before -22) all hold zero.
-template <typename T>
-static bool zero_from(const T *ring, int width, const qg_handle *h, int next)
-{
-  for(int i = 0; i < h->n_pad; ++i) {
-    const T *row = ring + (size_t)i * h->stride * width;
-    for(int k = next * width; k < (h->W - kWindow) * width; ++k)
-      if(row[k] != T(0)) return false;
-  }
-  return true;
-}
-
 extern "C" qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t bytes)
 {
   if(!h || !buf) return qg_fail(QG_ERR_INVALID_ARG, "qg_checkpoint_load: NULL argument");
@@ -2288,10 +2275,6 @@ extern "C" qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t by
   QG_CUDA(cudaSetDevice(h->device));
   for(int i = 0; i < qg_handle_s::kProfRing; ++i) QG_TRY(collect_prof(h, i));
   const char *p = static_cast<const char *>(buf) + sizeof hd;
-  const bool clean = zero_from(reinterpret_cast<const double *>(p), 2, h, hd.next_step) &&
-                     (!h->mixed || (zero_from(reinterpret_cast<const float *>(p + hd.ring_bytes), 2, h, hd.next_step) &&
-                                    zero_from(reinterpret_cast<const float *>(p + hd.ring_bytes + hd.ring32_bytes), 2,
-                                              h, hd.next_step)));
   QG_CUDA(cudaMemcpyAsync(h->d_ring, p, hd.ring_bytes, cudaMemcpyHostToDevice, h->stream));
   p += hd.ring_bytes;
   if(h->mixed) {
@@ -2303,11 +2286,20 @@ extern "C" qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t by
   QG_CUDA(cudaMemcpyAsync(h->d_pcr, p, hd.pcr_bytes, cudaMemcpyHostToDevice, h->stream));
   QG_CUDA(cudaMemcpyAsync(h->d_ints + 2, &hd.bad, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   QG_TRY(clear_flags(h));
+  // the slots from next_step on, which a run this early shares with the steps
+  // before -22: clean if all hold zero.  Later blocks read none of those.
+  int written = 1;
+  if(hd.next_step < h->max_delay + h->q - kWindow) {
+    QG_CUDA(cudaMemsetAsync(h->d_ints + 1, 0, sizeof(int), h->stream));
+    launch_ring_nonzero(h->step_args(false), hd.next_step, h->W - kWindow, h->d_ints + 1, h->stream);
+    QG_CUDA(cudaGetLastError());
+    QG_CUDA(cudaMemcpyAsync(&written, h->d_ints + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  }
   QG_CUDA(cudaStreamSynchronize(h->stream));
   h->next_step = hd.next_step;
   h->far_block = -0x7fffffff;
   h->eval_cached = -0x7fffffff;
-  h->ring_clean = clean;
+  h->ring_clean = written == 0;
   h->dev_next = -1;
   return QG_OK;
 }

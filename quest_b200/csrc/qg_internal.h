@@ -264,6 +264,8 @@ void launch_far_step1(const FarArgs &a, void *stream);
 void launch_far_batch(const FarArgs *args, const int *block_off, const int *tile_off, int n_ens, int blocks, int tiles,
                       int q, int frame, int mixed, int form, void *stream);
 void launch_ring32_rebuild(const StepArgs &a, void *stream);
+// *out = 1 if any ring (FP64, and FP32 in mixed precision) holds a non-zero in slots [lo, hi)
+void launch_ring_nonzero(const StepArgs &a, int lo, int hi, int *out, void *stream);
 // Sharded handles: a shard's rho01 at step t for internal dots [lo, hi)
 // into out[0 .. hi-lo), and the other dots' rho01 at step t from the full
 // internal-order vector into the rings (as the step kernel writes its own)

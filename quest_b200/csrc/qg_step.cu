@@ -1639,4 +1639,26 @@ void launch_ring32_rebuild(const StepArgs &a, void *stream)
   ring32_rebuild_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a);
 }
 
+// A NaN counts as written.
+__global__ void ring_nonzero_kernel(StepArgs a, int lo, int hi, int *out)
+{
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if(i >= (long long)a.n_pad * (hi - lo)) return;
+  const long long at = i / (hi - lo) * a.stride + lo + i % (hi - lo);
+  const double2 v = a.ring[at];
+  bool zero = v.x == 0.0 && v.y == 0.0;
+  if(a.ring32w) {
+    const float2 w = a.ring32w[at], d = a.ring32d[at];
+    zero = zero && w.x == 0.f && w.y == 0.f && d.x == 0.f && d.y == 0.f;
+  }
+  if(!zero) *out = 1;
+}
+
+void launch_ring_nonzero(const StepArgs &a, int lo, int hi, int *out, void *stream)
+{
+  if(lo >= hi) return;
+  const long long total = (long long)a.n_pad * (hi - lo);
+  ring_nonzero_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a, lo, hi, out);
+}
+
 }  // namespace qg

@@ -102,3 +102,31 @@ def test_both_forms_give_the_same_bits(golden_weights, mode, precision, frame, q
             outs.append(np.concatenate([first, sim.run(312)]))
     assert np.abs(outs[0][..., 1]).max() > 1e-8
     np.testing.assert_array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("precision,value", [(capi.PREC_FP64, 0.0), (capi.PREC_FP64, 1.0), (capi.PREC_FP64, np.nan),
+                                             (capi.PREC_MIXED, 0.0), (capi.PREC_MIXED, 1.0)])
+def test_a_checkpoint_brings_what_the_ring_holds(golden_weights, precision, value):
+    """A checkpoint taken early, with an iterate written into a slot the next
+    blocks' windows share with a step before -22: the loaded handle does not
+    take the slot for a zero unless it is one, and continues as one that was
+    never saved."""
+    wl = workload(300, 0, 5, 400)
+
+    def begin(early):
+        sim = capi.Simulation(wl.dots, wl.pulse, wl.constants, weights=golden_weights, precision=precision,
+                              coef_mode=capi.COEF_TABLE)
+        sim.set_option("far_early", early)
+        return sim
+
+    outs = []
+    for early in (1, 0):
+        with begin(early) as a, begin(early) as b:
+            a.run(32)
+            step = a.info()["ring_depth"] - 40  # step -40's slot
+            a.history_evaluate(step, np.full(a.n, value, dtype=np.complex128))
+            b.restore(a.checkpoint())
+            outs += [a.run(80), b.run(80)]
+    for o in outs[1:]:
+        np.testing.assert_array_equal(outs[0], o)
+    assert np.isfinite(outs[0]).all()
