@@ -58,18 +58,17 @@ Q = 5
 FALLBACK_HBM_GBS = 6650.0
 GOLDEN_WEIGHTS = os.path.join(ROOT, "tests", "golden", "pc_weights_18_22_3.15.txt")
 TABLE_BYTES_PER_PAIR = lambda q: 4 + 16 * (q + 1)  # noqa: E731  int32 delay + (q+1) complex128
-# FP64 flops of one on-the-fly coefficient evaluation (pair_coef_otf, q = 5):
-# 6 reciprocals + node products and sums (~190), dyad scalars (~30), 6 taps
-# of complex assembly (~90), sqrt / modf / sincos counted as ~40
-OTF_COEF_FLOPS = 350
-# Mixed precision (pair_coef_otf_mixed, q = 5): FP64 for the distance, the
-# delay split, 1/r and the phase reduction (~80, sqrt and divisions counted
-# as ~20 each); FP32 for the weights (6 nodes x (5 subtractions + 15 FMA of
-# the symmetric-polynomial recurrence + 6 products) ~ 250), the dyad scalars
-# (~35) and the 6 taps with their sum (~120).  Both are censuses of those
-# forms; the kernels' present forms take fewer operations, and the counts are
-# kept so that rates compare.
-OTF_COEF_FLOPS_MIXED = (80, 400)  # (FP64, FP32)
+# Operations of one on-the-fly coefficient evaluation at q = 5, rotating frame
+# (a fused multiply-add counts two; sqrt 20, a sine with its cosine 40 in FP64
+# and 20 in FP32).  FP64 (pair_geom, pair_coef_otf): separation and delay split
+# 34, dipole products and dyad scalars 34, phase and sincos 43, the three
+# factors 24, node reciprocals and sums 131, six taps 60.
+OTF_COEF_FLOPS = 326
+# Mixed precision (pair_coef_otf_mixed): FP64 for the separation and delay
+# split 34, 1/r 7 and the phase reduction 5; FP32 for the dipole products and
+# dyad scalars 27, sincos 20, the three factors 24, the node products with
+# their derivatives 85 and six taps 72.
+OTF_COEF_FLOPS_MIXED = (46, 228)  # (FP64, FP32)
 STEP_FORMS = {0: "general (1 launch per 16 steps)", 1: "fused (1 launch per step)",
               2: "block (1 cooperative launch per 16 steps)"}
 

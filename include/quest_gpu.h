@@ -224,9 +224,9 @@ qg_status qg_checkpoint_save(qg_handle *h, void *buf, size_t bytes);
 qg_status qg_checkpoint_load(qg_handle *h, const void *buf, size_t bytes);
 
 /* Batches: many independent ensembles (handles) advanced together, one
- * persistent far-pair launch and one step launch per step for all of them,
- * driven by an (ensemble, target tile, source-tile group) work list, the
- * 16-step block replayed as one CUDA graph.  No reference counterpart: the
+ * far-pair launch with its reduction per 16 steps and one step launch per step
+ * for all of them (a thread block finds its ensemble by a search over the
+ * members' offsets), the 16-step block replayed as one CUDA graph.  No reference counterpart: the
  * reference runs one ensemble per process.  Members keep their own device
  * state and are advanced exactly as qg_run would advance them (bitwise the
  * same results); they must share interpolation order, frame and history

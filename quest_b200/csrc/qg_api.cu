@@ -509,9 +509,9 @@ static int num_parts(int nT, int group)
 
 // Parts the partial buffer must hold: those of the handle's group, of the
 // on-the-fly group, and for table handles of up to 512 tiles of every group
-// the "far_group" option can set (those of group g are at most (nT / g + 1)
-// x 2 g, a part being 16 sources or more, and fewer than those of group 1
-// once 600 blocks need no cut).
+// the "far_group" option can set.  far_parts cuts a group of g tiles into 4 g
+// parts of 8 sources at the most, and not where two parts would already make
+// more than 1776 tasks; the largest number over the groups is taken as it is.
 static int max_parts(int nT, int group, bool otf)
 {
   int m = std::max(num_parts(nT, group), num_parts(nT, otf_group(nT)));
@@ -520,7 +520,7 @@ static int max_parts(int nT, int group, bool otf)
   return m;
 }
 
-// Even, so every ring row starts 32-byte aligned for paired-sample loads.
+// Even, so that every ring row starts at a 32-byte sector.
 static int ring_depth(int max_delay, int q)
 {
   const int w = max_delay + q + kTimeBlock + 2;

@@ -94,9 +94,9 @@ struct TableArgs {
 // What a far launch knows of its windows.  kFormAny: nothing; samples before
 // step -22 are skipped.  kFormPlain: no sample needs to be: every window starts
 // at step -22 or later (blocks past the largest delay), or every coefficient
-// is finite and the ring slots of steps before -22 still hold the zeros they
-// were reset to (the history was only ever written by the run itself), whose
-// products are +-0 and leave an accumulator that started at +0 bit for bit
+// is finite as it is held and the ring slots of steps before -22 still hold the
+// zeros they were reset to (nothing but runs has written the history, and no
+// captured call that would is about), whose products are +-0 and leave an accumulator that started at +0 bit for bit
 // as it was.  Both forms give the same bits.  The plain form serves the first
 // blocks too: testing or zeroing the dead samples there made a 640-step run
 // of 4096 dots 2-4 % slower than it began, and the tests' registers cost the
